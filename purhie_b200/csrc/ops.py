@@ -355,6 +355,9 @@ def sample_chain(logits: torch.Tensor, rows: torch.Tensor, out: torch.Tensor) ->
 register_signatures("core", {
     "ph_attention_generic_sink": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p],
+    "ph_attention_generic_capped": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p,
+                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
+                                    c_void_p, c_longlong, c_float, c_void_p],
     "ph_attention_talking": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_void_p,
                              c_void_p, c_void_p, c_int, c_longlong, c_void_p],

@@ -1,9 +1,11 @@
-"""The float32 product kernels give, bit for bit, what the plain kernels give: an operand that does not start
+"""The float32 product and attention kernels give, bit for bit, what the plain kernels give: an operand that does not start
 on 16 bytes goes to the plain kernel, whose additions run in the same order."""
+import math
+
 import pytest
 import torch
 
-from test_gpu_kernels import rnd
+from test_gpu_kernels import paged_case, rnd
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -32,3 +34,50 @@ def test_float32_product_adds_in_the_plain_kernels_order(M, N, K):
     # K products, each exact inside one rounded multiply-add: at most K half units in the last place of the sum of magnitudes
     bound = K * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)
     assert ((out.double() - x.double() @ w.double().T).abs() <= bound).all()
+
+
+# decoded tokens alone (rows kernel), portions long enough for tiles beside decoded tokens, a portion of three tokens, portions
+# that start mid-context; block edges of 32 and 128 keys; enough rows for tiles of eight rows a warp
+CASES = [[(1, 1), (32, 1), (33, 1), (128, 1), (129, 1), (300, 1)],
+         [(40, 40), (1, 1), (129, 1), (161, 33), (300, 3), (260, 5), (64, 32)],
+         [(2, 2), (35, 35), (1000, 20)],
+         [(1300, 1200)] + [(200 + i, 1) for i in range(20)]]
+
+
+@pytest.mark.parametrize("segs", CASES)
+@pytest.mark.parametrize("HQ,HKV,D,page_size,window,chunk", [(8, 2, 32, 16, None, 0), (4, 4, 64, 8, None, 0), (4, 2, 128, 16, None, 0),
+                                                             (8, 8, 128, 16, None, 0), (3, 1, 128, 5, None, 0), (4, 2, 128, 16, 50, 0),
+                                                             (2, 2, 64, 16, None, 48)])
+def test_float32_attention_adds_in_the_plain_kernels_order(segs, HQ, HKV, D, page_size, window, chunk):
+    from purhie_b200.csrc import ops
+    case = paged_case(segs, HQ, HKV, D, page_size, torch.float32, seed=3)
+    outs = []
+    for q in (case["q"], off_by_one(case["q"])):
+        out = torch.full((case["T"], HQ * D), float("nan"), device=DEV)
+        ops.attention_generic(q, case["k_base"], case["v_base"], case["page_stride"], page_size, case["table"], case["row_seg"],
+                              case["positions"], out, num_heads=HQ, num_kv_heads=HKV, head_dim=D, window=window,
+                              scale=1.0 / math.sqrt(D), chunk=chunk)
+        outs.append(out)
+    assert not torch.isnan(outs[0]).any()
+    assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("cap", [0.0, 2.0])
+@pytest.mark.parametrize("D", [32, 128])
+def test_float32_attention_with_sink_bias_gate_and_cap(D, cap):
+    from purhie_b200.csrc import ops
+    HQ, HKV, ps = 4, 2, 16
+    case = paged_case([(70, 40), (1, 1), (200, 1)], HQ, HKV, D, ps, torch.float32, seed=4)
+    sink, slopes, gate = rnd(HQ, seed=5), rnd(HQ, seed=6).abs() * 0.05, rnd(case["T"], HQ * D, seed=7)
+    if cap:
+        slopes = None
+    outs = []
+    for q in (case["q"], off_by_one(case["q"])):
+        out = torch.full((case["T"], HQ * D), float("nan"), device=DEV)
+        ops.call("core", "ph_attention_generic_capped", ops._ptr(q), ops._code(q.dtype), ops._ptr(case["k_base"]), ops._ptr(case["v_base"]),
+                 ops._code(torch.float32), case["page_stride"], ps, ops._ptr(case["table"]), case["table"].stride(0), ops._ptr(case["row_seg"]),
+                 ops._ptr(case["positions"]), ops._ptr(out), ops._code(torch.float32), case["T"], HQ, HKV, D, 0, 1.0 / math.sqrt(D), D, 0, 0,
+                 ops._ptr(sink), ops._ptr(slopes) if slopes is not None else None, ops._ptr(gate), HQ * D, cap, ops._stream())
+        outs.append(out)
+    assert not torch.isnan(outs[0]).any()
+    assert torch.equal(outs[0], outs[1])
