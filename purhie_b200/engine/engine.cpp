@@ -386,16 +386,20 @@ Tensor Engine::step_any(const std::vector<StepEntry>& entries, Layout& lay) {
 
 // A batch of single tokens: the launches of the whole model are captured once per (batch size, block table
 // widths, context bucket, what the parts added) and replayed.  Each graph owns its scratch memory and metadata
-// buffer, so nothing it points at ever moves.  The graph computes every row's logits; the wanted ones are picked
-// afterwards.
+// buffer, so nothing it points at ever moves.  The graph of a step that wants logits computes every row's; the wanted
+// ones are picked afterwards.  A step that wants none has a graph of its own, which ends behind the last layer: reading the
+// output matrix takes 0.2 ms at the 8B shape (eight layers, one row, eight steps of which one wants logits: 7.47 -> 6.08 ms)
+// and 0.06 ms at the 0.6B shape (28 layers: 9.25 -> 8.82 ms).
 Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* device_tokens, Layout& lay) {
     const int S = (int)entries.size();
     int need = 1;
     for (const StepEntry& e : entries)
         for (const PageGroup& g : cache_->groups()) need = std::max(need, (int)cache_->block_table(e.request, g.index).size() + 1);
-    layout(entries, pow2_at_least(need, 8), true, lay);
+    bool any_wanted = false;
+    for (const StepEntry& e : entries) any_wanted |= e.n_want > 0;
+    layout(entries, pow2_at_least(need, 8), any_wanted, lay);
     const int ctx_bucket = pow2_at_least(lay.decode_max_ctx, 256);
-    std::string key = std::to_string(S) + "|" + std::to_string(ctx_bucket);
+    std::string key = std::to_string(S) + "|" + std::to_string(ctx_bucket) + (any_wanted ? "|logits" : "");
     for (int w : lay.widths) key += "|w" + std::to_string(w);
     for (const auto& a : lay.extra) key += "|" + a.first + ":" + std::to_string(a.second.second);
     Graph* g = nullptr;
@@ -430,13 +434,13 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
             ctx.decode_max_ctx = ctx_bucket;                         // the number of attention splits must not change between replays
             // the first time: run the launches directly (this is the step's result, and whatever a kernel sets up
             // on first use is set up), then capture the same launches for the next time
-            g->logits = forward(ctx, rows, S);
+            g->logits = forward(ctx, rows, any_wanted ? S : 0);
             g->workspace.frozen = true;
             const long long before = g_launches;
             QE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeRelaxed));
             cudaGraph_t graph = nullptr;
             try {
-                forward(ctx, rows, S);
+                forward(ctx, rows, any_wanted ? S : 0);
             } catch (...) {
                 cudaStreamEndCapture(stream_, &graph);
                 if (graph) cudaGraphDestroy(graph);
@@ -460,11 +464,11 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
         if (g && !g->exec) graphs_.pop_back();                        // a graph that was never finished is not kept
         throw;
     }
+    if (!any_wanted) return Tensor();
     // pick the wanted rows
     std::vector<int> want;
     for (int s = 0; s < S; s++) if (entries[s].n_want) want.push_back(s);
     if ((int)want.size() == S) return g->logits;
-    if (want.empty()) return Tensor();
     const int64_t V = g->logits.shape[1];
     Tensor picked = workspace_.get("logits_picked", {(int64_t)want.size(), V}, DType::F32);
     for (size_t i = 0; i < want.size(); i++)
