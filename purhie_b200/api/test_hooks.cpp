@@ -399,6 +399,23 @@ API const char* qe_profile_report(int reset) {
     return guarded_text([&] { return LaunchProfile::get().report_json(reset != 0); });
 }
 
+// Page-locked memory for a result of `bytes`: its address in *data and a handle for qe_rows_give, or null when there is none
+// to be had (the caller then uses memory of its own).
+API void* qe_rows_take(inference_model_t* m, long long bytes, void** data) {
+    RowPool::Block* block = nullptr;
+    guarded([&] {
+        if (bytes > 0 && data) block = RowPool::take(need_engine(m).row_pool(), (size_t)bytes);
+        if (block) *data = block->memory.data();
+        return 0;
+    });
+    return block;
+}
+API void qe_rows_give(void* block) {
+    guarded([&] {
+        if (block) RowPool::give(static_cast<RowPool::Block*>(block));
+        return 0;
+    });
+}
 API long long qe_launches(void) { return g_launches; }
 API void qe_set_library_dir(const char* dir) { set_library_dir(dir ? dir : ""); }
 

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import json
+import weakref
 from ctypes import POINTER, c_float, c_int32
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
@@ -17,6 +18,12 @@ import numpy as np
 
 from .. import native
 from ..native import KernelError, OutOfPages, OutOfSlots, StepError
+
+
+# the C library's entry (native.StepEntryC), to be filled column by column
+_ENTRY = np.dtype([("request", np.int64), ("tokens", np.uint64), ("n_tokens", np.int32), ("want", np.uint64), ("n_want", np.int32)], align=True)
+assert _ENTRY.itemsize == ctypes.sizeof(native.StepEntryC)
+_POOLED_BYTES = 2 << 20                  # results from here on go into page-locked blocks; below, ordinary memory is as fast
 
 
 @dataclass
@@ -159,37 +166,66 @@ class Engine:
             return None
         batch, keep, wanted = self._batch(entries)
         out = native.StepOutputC()
-        logits = np.empty((max(wanted, 1), self.vocab_size), dtype=np.float32)
-        out.logits = logits.ctypes.data_as(POINTER(c_float))
+        logits = self._rows(wanted)
+        out.logits = ctypes.cast(logits.ctypes.data, POINTER(c_float))
         out.logits_capacity = logits.size
         native.check(native.lib().engine_step(self._handle, ctypes.byref(batch), ctypes.byref(out)))
         self.last_stats = StepStats(out.tokens, out.prompt_rows, out.decode_rows, out.n_rows, bool(out.replayed_graph))
         return logits[:out.n_rows] if out.n_rows else None
 
+    def _rows(self, wanted: int) -> np.ndarray:
+        """Memory for ``wanted`` rows of logits: several rows in a page-locked block that goes back to the engine's pool
+        when the array and its views are gone, else (or when the pool has none) ordinary memory."""
+        shape = (wanted, self.vocab_size)
+        if wanted * self.vocab_size * 4 >= _POOLED_BYTES:
+            data = ctypes.c_void_p()
+            block = native.lib().qe_rows_take(self._handle, wanted * self.vocab_size * 4, ctypes.byref(data))
+            if block:
+                held = (c_float * (wanted * self.vocab_size)).from_address(data.value)
+                weakref.finalize(held, native.lib().qe_rows_give, block).atexit = False
+                return np.frombuffer(held, dtype=np.float32).reshape(shape)
+        return np.empty(shape, dtype=np.float32)
+
     def _batch(self, entries):
-        """The C batch for ``entries`` (and the arrays it points into, which the caller keeps alive)."""
+        """The C batch for ``entries`` (and the arrays it points into, which the caller keeps alive).  A decoded token
+        given as a plain list of one int goes into one shared array: arrays of its own cost 10 us an entry."""
         seen = set()
         for e in entries:
             if e.request_id in seen:
                 raise StepError(f"request {e.request_id!r} is in the batch twice")
             seen.add(e.request_id)
-        arr = (native.StepEntryC * len(entries))()
-        keep = [arr]
+        n = len(entries)
+        rows = np.zeros(n, dtype=_ENTRY)
+        singles, tokens, counts, ids = [], [0] * n, [1] * n, []
+        keep = [rows]
         wanted = 0
         for i, e in enumerate(entries):
-            toks = np.ascontiguousarray(np.asarray(e.tokens, dtype=np.int64))
-            if toks.size and (toks.min() < -2**31 or toks.max() >= 2**31):
-                raise StepError(f"request {e.request_id!r}: a token id does not fit 32 bits")
-            toks = toks.astype(np.int32)
-            want = np.ascontiguousarray(np.asarray(list(e.want), dtype=np.int32))
-            keep.append((toks, want))
-            arr[i].request = self._id(e.request_id)
-            arr[i].tokens = toks.ctypes.data_as(POINTER(c_int32))
-            arr[i].n_tokens = int(toks.size)
-            arr[i].want = want.ctypes.data_as(POINTER(c_int32))
-            arr[i].n_want = int(want.size)
-            wanted += int(want.size)
-        return native.StepBatchC(arr, len(entries)), keep, wanted
+            given = e.tokens
+            if type(given) is list and len(given) == 1 and type(given[0]) is int:
+                if not -2**31 <= given[0] < 2**31:
+                    raise StepError(f"request {e.request_id!r}: a token id does not fit 32 bits")
+                tokens[i] = -len(singles) - 1                # its place in the shared array, whose address is not known yet
+                singles.append(given[0])
+            else:
+                toks = np.ascontiguousarray(np.asarray(given, dtype=np.int64))
+                if toks.size and (toks.min() < -2**31 or toks.max() >= 2**31):
+                    raise StepError(f"request {e.request_id!r}: a token id does not fit 32 bits")
+                toks = toks.astype(np.int32)
+                keep.append(toks)
+                tokens[i], counts[i] = toks.ctypes.data, int(toks.size)
+            if not (type(e.want) in (list, tuple) and not e.want):
+                want = np.ascontiguousarray(np.asarray(list(e.want), dtype=np.int32))
+                keep.append(want)
+                rows[i]["want"], rows[i]["n_want"] = want.ctypes.data, int(want.size)
+                wanted += int(want.size)
+            ids.append(self._id(e.request_id))
+        if singles:
+            shared = np.array(singles, dtype=np.int32)
+            keep.append(shared)
+            at = shared.ctypes.data
+            tokens = [t if t >= 0 else at + 4 * (-t - 1) for t in tokens]
+        rows["request"], rows["tokens"], rows["n_tokens"] = ids, tokens, counts
+        return native.StepBatchC(ctypes.cast(rows.ctypes.data, POINTER(native.StepEntryC)), n), keep, wanted
 
     # ---- timing on the device (the benchmark's) ------------------------------------------------------------------
     def time_step(self, entries: Sequence[StepEntry]) -> float:

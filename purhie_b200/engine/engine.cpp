@@ -511,6 +511,46 @@ void Engine::read_logits(const Tensor& logits, float* host) {
     check_kernel_errors();
 }
 
+RowPool::Block* RowPool::take(const std::shared_ptr<RowPool>& pool, size_t bytes) {
+    std::unique_ptr<Block> block;
+    {
+        std::lock_guard<std::mutex> lock(pool->mutex_);
+        // the smallest free block that holds it and is not more than twice as large
+        size_t best = pool->free_.size();
+        for (size_t i = 0; i < pool->free_.size(); i++) {
+            const size_t n = pool->free_[i]->memory.bytes();
+            if (n >= bytes && n / 2 <= bytes && (best == pool->free_.size() || n < pool->free_[best]->memory.bytes())) best = i;
+        }
+        if (best < pool->free_.size()) {
+            block = std::move(pool->free_[best]);
+            pool->free_.erase(pool->free_.begin() + best);
+        } else {
+            while (pool->held_ + bytes > kMost && !pool->free_.empty()) {        // blocks of other sizes make room
+                pool->held_ -= pool->free_.front()->memory.bytes();
+                pool->free_.erase(pool->free_.begin());
+            }
+            if (pool->held_ + bytes > kMost) return nullptr;
+            block.reset(new Block());
+            try {
+                block->memory.ensure(bytes);
+            } catch (const Error&) {                                             // no page-locked memory left: ordinary memory serves
+                cudaGetLastError();
+                return nullptr;
+            }
+            pool->held_ += block->memory.bytes();
+        }
+    }
+    block->pool = pool;
+    return block.release();
+}
+
+void RowPool::give(Block* given) {
+    std::unique_ptr<Block> block(given);
+    const std::shared_ptr<RowPool> pool = std::move(block->pool);
+    std::lock_guard<std::mutex> lock(pool->mutex_);
+    pool->free_.push_back(std::move(block));
+}
+
 // ---- sampling --------------------------------------------------------------------------------------------------------------
 PendingTokens* Engine::sample_async(const Tensor& logits, const std::vector<Sampler*>& samplers) {
     const int R = (int)samplers.size();

@@ -208,6 +208,8 @@ _SIGNATURES = {
     "qe_profile_enable": (None, [c_int]),
     "qe_profile_enabled": (c_int, []),
     "qe_profile_report": (c_char_p, [c_int]),
+    "qe_rows_take": (c_void_p, [_P, c_longlong, POINTER(c_void_p)]),
+    "qe_rows_give": (None, [c_void_p]),
     "qe_launches": (c_longlong, []),
     "qe_set_library_dir": (None, [c_char_p]),
 }

@@ -31,3 +31,26 @@ def test_steps_with_and_without_wanted_logits_give_the_same_logits(config, dtype
         results.append(np.stack(kept))
         eng.close()
     assert results[0].shape == results[1].shape and np.array_equal(results[0], results[1])
+
+
+def test_results_that_are_kept_stay_as_they_are():
+    """Several rows of logits lie in page-locked blocks of the engine's pool (64 MiB at most): results that are held, more of
+    them than the pool gives, are not touched by later steps, also when dropped ones have given their blocks back."""
+    from purhie_b200.engine import Engine, StepEntry
+    config = dict(TINY_C, vocab_size=400000, tie_word_embeddings=True)
+    eng = Engine.from_random(config, 3, dtype="bfloat16", page_size=16, max_tokens=2048, max_requests=2)
+    eng.add_request("a")
+    toks = random_tokens(160, config["vocab_size"], 5)
+    held, copies = [], []
+    for k in range(0, 160, 8):                        # 8 rows of 1.6 MB
+        out = eng.step([StepEntry("a", toks[k:k + 8], range(8))])
+        if k % 32 == 8:
+            del out
+            continue
+        held.append(out[2:])                          # (a view keeps its block)
+        copies.append(out[2:].copy())
+        del out
+    eng.close()
+    for a, b in zip(held, copies):
+        assert np.array_equal(a, b)
+    assert len({a.ctypes.data for a in held}) == len(held)
