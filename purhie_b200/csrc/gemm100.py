@@ -85,7 +85,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swapped: bool, 
     """out[M, N] = x[M, K] @ w[N, K]^T (out [splits, M, N] float32 partial sums when splits > 1).  With
     ``swiglu`` the rows of w are (gate, up) pairs and out is [M, N / 2] = silu(gate) * up.  ``accumulate``
     (plain orientation, float32, one split): out += the product.  ``row_sumsq`` [M, chunks] (swapped with bfloat16
-    out, or plain with block_n 256): the rows of x lack the factor rsqrt(sum(row_sumsq[m]) / row_width + row_eps);
+    out, or plain with block_n 64, 128 or 256): the rows of x lack the factor rsqrt(sum(row_sumsq[m]) / row_width + row_eps);
     the epilogue applies it.  ``norm_ahead`` (weight float32 [N], rows bfloat16 [M, N], sumsq float32 [M, 2 * ceil(N / 256)];
     plain, block_n 256, accumulate): rows = (the new out) * weight, sumsq[m, j] = the sum of squares of the new out
     over columns 128 j .. 128 j + 127."""

@@ -471,7 +471,9 @@ __device__ __forceinline__ void store_chunk_swapped_bf16(const GemmParams& p, ui
     __syncwarp();                                      // the buffer is written again for the next chunk
 }
 
-template <int BN>
+// ROW_SCALE: the instance whose plain epilogue knows a factor per row (a register or two that the few-token instances of 64 and
+// 128 columns do without).
+template <int BN, bool ROW_SCALE>
 __global__ void __launch_bounds__(NUM_THREADS, TileConfig<BN>::CTAS_PER_SM)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmParams p) {
     using Cfg = TileConfig<BN>;
@@ -531,17 +533,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             wa.start(blockIdx.x, work_total);
             wb.start(blockIdx.x, work_total);
             int pre = 0;
-            if (p.swapped) {
-                // A is the weight: fill the (still empty) ring with weight tiles now
-                for (; pre < STAGES && wa.valid; ++pre) {
-                    mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
-                    tma_load_2d(smem_a + pre * A_BYTES, &map_a, &full[pre], wa.kb * BK, wa.a0);
-                    wa.next(gridDim.x, work_total);
-                }
+            // fill the (still empty) ring with tiles of the weight now: A in the swapped orientation, B in the plain one
+            for (; pre < STAGES && wa.valid; ++pre) {
+                mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
+                if (p.swapped) tma_load_2d(smem_a + pre * A_BYTES, &map_a, &full[pre], wa.kb * BK, wa.a0);
+                else tma_load_2d(smem_b + pre * Cfg::B_BYTES, &map_b, &full[pre], wa.kb * BK, wa.b0);
+                wa.next(gridDim.x, work_total);
             }
             pdl_wait();
             for (int s = 0; s < pre; ++s) {                  // the activation tiles of those stages
-                tma_load_2d(smem_b + s * Cfg::B_BYTES, &map_b, &full[s], wb.kb * BK, wb.b0);
+                if (p.swapped) tma_load_2d(smem_b + s * Cfg::B_BYTES, &map_b, &full[s], wb.kb * BK, wb.b0);
+                else tma_load_2d(smem_a + s * A_BYTES, &map_a, &full[s], wb.kb * BK, wb.a0);
                 wb.next(gridDim.x, work_total);
             }
             int stage = pre == STAGES ? 0 : pre;
@@ -616,14 +618,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     factor[i] = rsqrtf(s / (float)p.row_width + p.row_eps);
                 }
             }
-            // plain orientation, tiles of 256 columns: the factor of this thread's row (fetched while the products run), and
-            // its sum of squares for the norm ahead
+            // plain orientation: the factor of this thread's row (fetched while the products run), and its sum of squares for
+            // the norm ahead (tiles of 256 columns)
             const int a = a0 + q * 32 + lane;
             constexpr bool ROW_OPS = BN == 256;
-            const bool scale_row = ROW_OPS && !p.swapped && p.row_sumsq != nullptr;
+            const bool scale_row = ROW_SCALE && !p.swapped && p.row_sumsq != nullptr;
             float row_f = 1.0f;
             float ss[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if constexpr (ROW_OPS) row_f = scale_row ? plain_row_factor(p, a) : 1.0f;
+            if constexpr (ROW_SCALE) row_f = scale_row ? plain_row_factor(p, a) : 1.0f;
             if (!mbar_wait(&acc_full[acc], acc_phase, p.error_flag, PH_ERR_WAIT_EPILOGUE)) { ok = false; break; }
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
@@ -644,7 +646,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
                 if constexpr (CH == 32) tmem_ld32(taddr + c, r); else tmem_ld16(taddr + c, r);
                 tmem_ld_wait();
-                if constexpr (ROW_OPS) {
+                if constexpr (ROW_SCALE) {
                     if (scale_row) {
 #pragma unroll
                         for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * row_f);
@@ -753,8 +755,9 @@ __device__ __forceinline__ void put_chunk(unsigned char* box, int lane, int chun
     *(uint4*)(box + lane * 128 + ((chunk ^ (lane & 7)) << 4)) =
         make_uint4(*(const uint32_t*)&a, *(const uint32_t*)&b, *(const uint32_t*)&c, *(const uint32_t*)&d);
 }
-__device__ __forceinline__ float silu_times(const GemmParams& p, uint32_t g_bits, uint32_t u_bits, float f) {
-    return gate_times(p, __uint_as_float(g_bits) * f, __uint_as_float(u_bits) * f);
+// beside: 0, or 1 in a lane whose row lies behind the last one, which would otherwise divide zeros (see `live`).
+__device__ __forceinline__ float silu_times(const GemmParams& p, uint32_t g_bits, uint32_t u_bits, float f, float beside) {
+    return gate_times(p, fmaf(__uint_as_float(g_bits), f, beside), __uint_as_float(u_bits) * f);
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -903,10 +906,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 // clipped by the copy
                 unsigned char* box = (unsigned char*)(staging + (warp - 2) * 32 * 32);
                 const int row0 = a0 + q * 32;
+                // A warp whose rows all lie behind the last one has nothing to work out: its zeros sent the activation's division
+                // down a slow path (128 x 6144 x 1024, half a row tile: 22.6 us, 16.0 without)
+                const bool live = row0 < p.rows_a;
+                const float beside = a < p.rows_a ? 0.0f : 1.0f;
                 if (p.tma_store == 2) {
                     // float32: every chunk of 32 accumulator columns is a box
 #pragma unroll 1
-                    for (int c = c_first; c < c_first + PAIR_BN / 2; c += 32) {
+                    for (int c = c_first; live && c < c_first + PAIR_BN / 2; c += 32) {
                         uint32_t r[32];
                         tmem_ld32(taddr + c, r);
                         if (lane == 0) tma_store_wait_read();
@@ -919,7 +926,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                                             __uint_as_float(r[4 * j + 2]) * row_f, __uint_as_float(r[4 * j + 3]) * row_f);
                         fence_async_shared();
                         __syncwarp();
-                        if (lane == 0 && row0 < p.rows_a && b0 + c < p.rows_b) tma_store_3d(&map_out, box, b0 + c, row0, w % p.splits);
+                        if (lane == 0 && b0 + c < p.rows_b) tma_store_3d(&map_out, box, b0 + c, row0, w % p.splits);
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -927,7 +934,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     if (++acc == 2) { acc = 0; acc_phase ^= 1; }
                     continue;
                 }
-                const int boxes = p.swiglu ? 1 : 2, per_box = p.swiglu ? 4 : 2;       // chunks of 32 accumulator columns per box
+                const int boxes = !live ? 0 : p.swiglu ? 1 : 2, per_box = p.swiglu ? 4 : 2;       // chunks of 32 accumulator columns per box
 #pragma unroll 1
                 for (int b = 0; b < boxes; ++b) {
                     if (lane == 0) tma_store_wait_read();                          // the box before this one has left shared memory
@@ -941,10 +948,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 #pragma unroll
                             for (int j = 0; j < 2; ++j)
                                 put_chunk(box, lane, 2 * k + j,
-                                          silu_times(p, r[16 * j], r[16 * j + 1], row_f), silu_times(p, r[16 * j + 2], r[16 * j + 3], row_f),
-                                          silu_times(p, r[16 * j + 4], r[16 * j + 5], row_f), silu_times(p, r[16 * j + 6], r[16 * j + 7], row_f),
-                                          silu_times(p, r[16 * j + 8], r[16 * j + 9], row_f), silu_times(p, r[16 * j + 10], r[16 * j + 11], row_f),
-                                          silu_times(p, r[16 * j + 12], r[16 * j + 13], row_f), silu_times(p, r[16 * j + 14], r[16 * j + 15], row_f));
+                                          silu_times(p, r[16 * j], r[16 * j + 1], row_f, beside), silu_times(p, r[16 * j + 2], r[16 * j + 3], row_f, beside),
+                                          silu_times(p, r[16 * j + 4], r[16 * j + 5], row_f, beside), silu_times(p, r[16 * j + 6], r[16 * j + 7], row_f, beside),
+                                          silu_times(p, r[16 * j + 8], r[16 * j + 9], row_f, beside), silu_times(p, r[16 * j + 10], r[16 * j + 11], row_f, beside),
+                                          silu_times(p, r[16 * j + 12], r[16 * j + 13], row_f, beside), silu_times(p, r[16 * j + 14], r[16 * j + 15], row_f, beside));
                         } else {
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
@@ -957,7 +964,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     fence_async_shared();
                     __syncwarp();
                     const int col0 = p.swiglu ? (b0 + c_first) >> 1 : b0 + c_first + b * 64;
-                    if (lane == 0 && row0 < p.rows_a && col0 < (int)p.ld) tma_store_2d(&map_out, box, col0, row0);
+                    if (lane == 0 && col0 < (int)p.ld) tma_store_2d(&map_out, box, col0, row0);
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -1095,11 +1102,11 @@ int sm_count() {
     return n;
 }
 
-template <int BN>
+template <int BN, bool ROW_SCALE>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int max_ctas, cudaStream_t stream) {
     using Cfg = TileConfig<BN>;
     static bool configured = false;
-    auto kernel = gemm_tcgen05_kernel<BN>;
+    auto kernel = gemm_tcgen05_kernel<BN, ROW_SCALE>;
     if (!configured) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
             return fail(PH_ERR_LAUNCH, "gemm_tcgen05: cannot reserve %d bytes of shared memory", Cfg::SMEM_BYTES);
@@ -1267,8 +1274,10 @@ PH_EXPORT int ph_gemm_bf16_tcgen05(const void* x, const void* w, void* out, int 
     if (row_sumsq && swapped && (out_dtype != PH_BF16 || splits > 1 || row_chunks < 1 || row_width < 1))
         return fail(PH_ERR_ARG, "gemm_tcgen05: in the swapped orientation a factor per token goes with bfloat16 output and one split");
     if (!swapped) {
-        if ((row_sumsq || norm_weight || norm_rows || norm_sumsq) && block_n != 256)
-            return fail(PH_ERR_ARG, "gemm_tcgen05: in the plain orientation the row operations go with tiles of 256 columns");
+        if ((norm_weight || norm_rows || norm_sumsq) && block_n != 256)
+            return fail(PH_ERR_ARG, "gemm_tcgen05: in the plain orientation the rows for the norm ahead go with tiles of 256 columns");
+        if (row_sumsq && block_n < 64)
+            return fail(PH_ERR_ARG, "gemm_tcgen05: in the plain orientation a factor per token goes with tiles of 64 columns or more");
         if (const char* why = row_ops_refused(row_sumsq, row_chunks, row_width, norm_weight, norm_rows, norm_sumsq, splits, accumulate, N))
             return fail(PH_ERR_ARG, "gemm_tcgen05: %s", why);
     } else if (norm_weight || norm_rows || norm_sumsq) {
@@ -1291,12 +1300,13 @@ PH_EXPORT int ph_gemm_bf16_tcgen05(const void* x, const void* w, void* out, int 
     p.row_sumsq = row_sumsq; p.row_chunks = row_chunks; p.row_width = row_width; p.row_eps = row_eps;
     p.norm_weight = norm_weight; p.norm_rows = (__nv_bfloat16*)norm_rows; p.norm_sumsq = norm_sumsq;
     p.tma_store = 0;
+    const bool scaled = !swapped && row_sumsq != nullptr;
     switch (block_n) {
-        case 16: return launch<16>(ma, mb, p, max_ctas, stream);
-        case 32: return launch<32>(ma, mb, p, max_ctas, stream);
-        case 64: return launch<64>(ma, mb, p, max_ctas, stream);
-        case 128: return launch<128>(ma, mb, p, max_ctas, stream);
-        case 256: return launch<256>(ma, mb, p, max_ctas, stream);
+        case 16: return launch<16, false>(ma, mb, p, max_ctas, stream);
+        case 32: return launch<32, false>(ma, mb, p, max_ctas, stream);
+        case 64: return scaled ? launch<64, true>(ma, mb, p, max_ctas, stream) : launch<64, false>(ma, mb, p, max_ctas, stream);
+        case 128: return scaled ? launch<128, true>(ma, mb, p, max_ctas, stream) : launch<128, false>(ma, mb, p, max_ctas, stream);
+        case 256: return launch<256, true>(ma, mb, p, max_ctas, stream);
         default: return fail(PH_ERR_ARG, "gemm_tcgen05: block_n %d is not one of 16, 32, 64, 128, 256", block_n);
     }
 }

@@ -29,29 +29,38 @@ GemmPlan plan_few(int M, int N, int K, int sms, bool allow_split) {
     return p;
 }
 
-// Many tokens, plain orientation: the one-CTA kernel (tiles of 128 tokens x 256 features) or the pair kernel
-// (256 x 256 on two SMs), and into how many parts K is cut.  Estimated cost in units of one block of K on one
-// SM's tile: rounds of the CTAs (or pairs) times the item's blocks (the pair spends 0.87 of a block's time per
-// block: half the shared-memory traffic per flop) plus six for an item's start and epilogue, plus the float32
-// partial results' way to memory and back when K is split.  A fused epilogue needs the whole sum in one place.
+// Many tokens, plain orientation: tiles of 128 tokens x 64, 128 or 256 features on one CTA, or of 256 x 256 on a pair of SMs,
+// and into how many parts K is cut.  Estimated microseconds, fitted to products of 128 to 2,048 tokens with 1,024 to 16,384
+// features and K 1,024 to 8,192: what a launch costs (the pair kernel does not start early), plus rounds of the CTAs times a
+// round's blocks of K, start and epilogue (longer with an activation), plus the float32 partial results' way to memory and
+// back when K is split.  A fused epilogue needs the whole sum in one place.  The narrow tiles are for products whose wide
+// tiles would leave most SMs without one: 256 x 6144 x 1024 with the activation 11.1 us with tiles of 64 columns, 20.1 with
+// 256, 16.0 on pairs; 544 x 1024 x 2048 8.1 us with tiles of 128 and three parts of K, 9.6 on pairs with six; 544 x 4096 x 1024
+// 10.4 us with tiles of 256 on one CTA, 11.6 on pairs.  A long K that stays whole without an activation keeps the wide tiles:
+// by itself 1024 x 2048 x 2048 takes 14.2 us with tiles of 128 and 16.7 on pairs, in a model's chain of launches it was no
+// faster (15 us of 2,060 slower for a prompt of a model of that width).
 void plan_many(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue, GemmPlan& p) {
     const int kblocks = ceil_div(K, kBlockK);
     static const int kAll[] = {1, 2, 3, 4, 6, 8};
+    struct Kind { bool pair; int bn, per_sm; double launch, block, item, activation; };
+    static const Kind kKinds[] = {{false, 256, 1, 1.8, 0.31, 5.0, 6.0}, {true, 256, 0, 4.5, 0.28, 3.0, 4.5},
+                                  {false, 128, 1, 1.8, 0.255, 2.2, 4.5}, {false, 64, 2, 1.8, 0.28, 2.0, 0.5}};
     const int n_options = (allow_split && !fused_epilogue) ? 6 : 1;
     double best = -1.0;
     p.pair = false;
     p.splits = 1;
-    for (int pair = 0; pair < 2; pair++) {
-        if (pair && (M <= 128 || N <= 128)) continue;
-        const int tiles = (pair ? ceil_div(M, 256) : ceil_div(M, 128)) * ceil_div(N, 256);
-        const int slots = pair ? sms / 2 : sms;
+    for (const Kind& k : kKinds) {
+        if (k.pair && (M <= 128 || N <= 128)) continue;
+        const int tiles = ceil_div(M, k.pair ? 256 : 128) * ceil_div(N, k.bn);
+        const int slots = k.pair ? sms / 2 : sms * k.per_sm;
         for (int o = 0; o < n_options; o++) {
             const int s = kAll[o];
-            if (s > 1 && kblocks / s < 8) continue;
+            if (s > 1 && (kblocks / s < 8 || k.bn == 64)) continue;
+            if (s == 1 && n_options > 1 && k.bn < 256 && kblocks >= 32) continue;
             const int rounds = ceil_div((long long)tiles * s, slots);
-            double cost = rounds * ((pair ? 0.87 : 1.0) * kblocks / s + 6.0);
-            if (s > 1) cost += 2.0 * s * (double)M * N * 4 / 4.0e12 / 0.33e-6;
-            if (best < 0 || cost < best - 1e-9) { best = cost; p.pair = pair != 0; p.splits = s; }
+            double cost = k.launch + rounds * (k.block * kblocks / s + k.item + (fused_epilogue ? k.activation : 0.0));
+            if (s > 1) cost += 2.0 * s * (double)M * N * 4 / 4.0e6;
+            if (best < 0 || cost < best - 1e-9) { best = cost; p.pair = k.pair; p.splits = s; p.block_n = k.bn; }
         }
     }
 }
@@ -94,8 +103,8 @@ bool Linear::applies_row_scale(int rows, DType out_dtype, bool fuse_swiglu, bool
     const GemmPlan p = plan_gemm(rows, (int)weight_.shape[0], (int)weight_.shape[1], sm_count(), allow_split, fused);
     // few rows: the fused activation keeps K whole and writes bfloat16 from the swapped epilogue, which is where the factor goes
     if (p.swapped) return out_dtype == DType::BF16 && fused;
-    // many rows: the epilogue of the 256-feature tiles, whenever it holds whole sums
-    return p.block_n == 256 && p.splits == 1;
+    // many rows: the epilogue of tiles of 64 features and more, whenever it holds whole sums
+    return p.block_n >= 64 && p.splits == 1;
 }
 
 bool Linear::gives_partial_sums(int rows, bool allow_split) const {
@@ -154,6 +163,11 @@ Addend Linear::operator()(const Tensor& x_in, StepContext& ctx, const std::strin
     const GemmKernels& g = gemm_kernels();
     const bool fused = fuse_swiglu && N % 2 == 0;
     GemmPlan p = plan_gemm(M, N, K, sm_count(), allow_split, fused);
+    if (add_into && ctx.residual_width == N && ahead && ahead->offered() && !p.swapped && p.splits == 1 && p.block_n < 256 && N > 128) {
+        // the epilogue of wide tiles also does the next norm's work, which saves the norm's launch behind narrow ones
+        p.block_n = 256;
+        p.pair = M > 128;          // 1024 x 2048 x 2048 with the addition: 18.9 us, 23.9 on one CTA
+    }
     auto run = [&](Tensor& out, int splits, bool swiglu, bool accumulate, NormAhead* work_ahead = nullptr) {
         if (LaunchProfile::get().on())      // what the product has to move and to compute: the weight once, x, and its result
             LaunchProfile::get().note_cost(2.0 * N * K + 2.0 * M * K + (double)out.bytes(), 2.0 * M * N * K);

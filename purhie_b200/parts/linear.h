@@ -50,7 +50,7 @@ public:
     // swapped).  Its partial sums are linear in the rows, and its bfloat16 epilogue can apply a factor per row.
     bool swapped_for(int rows, bool allow_split, bool fused_epilogue) const;
     // The product's own epilogue multiplies by the rows' factor: few rows with the fused activation; many rows
-    // (tiles of 256 features) whenever K stays whole and nothing is added into the output.
+    // (tiles of 64 features and more) whenever K stays whole and nothing is added into the output.
     bool applies_row_scale(int rows, DType out_dtype, bool fuse_swiglu, bool allow_split = true) const;
     // Many rows, K cut into parts: float32 partial sums, linear in the rows, so whoever adds them up can apply the factor.
     bool gives_partial_sums(int rows, bool allow_split) const;

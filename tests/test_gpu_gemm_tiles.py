@@ -1,0 +1,53 @@
+"""Plain tiles of 64, 128 and 256 columns with the factor per row, and ragged row tiles of the pair kernel."""
+import pytest
+import torch
+
+from test_gpu_kernels import rel, rnd
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def scaled_case(M, N, K, chunks=3, eps=1e-6):
+    x, w = rnd(M, K, dtype=torch.bfloat16, seed=31), rnd(N, K, dtype=torch.bfloat16, seed=32, scale=0.2)
+    sumsq = rnd(M, chunks, seed=33).abs() + 0.1
+    factor = torch.rsqrt(sumsq.double().sum(1) / K + eps)
+    return x, w, sumsq, (x.double() @ w.double().T) * factor[:, None]
+
+
+@pytest.mark.parametrize("M", [128, 129, 517, 1100])
+@pytest.mark.parametrize("N,K", [(192, 128), (520, 200)])
+@pytest.mark.parametrize("kernel", [64, 128, 256, "pair"])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_rows_without_their_factor(M, N, K, kernel, swiglu):
+    from purhie_b200.csrc import gemm100
+    x, w, sumsq, y = scaled_case(M, N, K)
+    ref = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2] if swiglu else y
+    kw = dict(swiglu=swiglu, row_sumsq=sumsq, row_width=K, row_eps=1e-6)
+    for dtype, bound in ((torch.float32, 2e-5), (torch.bfloat16, 5e-3)):     # sums in float32; a bfloat16 result is rounded once
+        out = torch.full((M, N // 2 if swiglu else N), float("nan"), dtype=dtype, device=DEV)
+        if kernel == "pair":
+            gemm100.gemm_pair(x, w, out, **kw)
+        else:
+            gemm100.gemm(x, w, out, swapped=False, block_n=kernel, **kw)
+        gemm100.check_errors(DEV)
+        assert not torch.isnan(out).any()
+        assert rel(out, ref) < bound
+
+
+@pytest.mark.parametrize("M", [257, 300, 513, 640])
+def test_pair_kernel_leaves_what_lies_behind_its_rows_alone(M):
+    """Warps whose rows lie behind the last one skip their epilogue: float32, partial sums, bfloat16 and the addition."""
+    from purhie_b200.csrc import gemm100
+    N, K = 384, 256
+    x, w = rnd(M, K, dtype=torch.bfloat16, seed=41), rnd(N, K, dtype=torch.bfloat16, seed=42)
+    ref = x.double() @ w.double().T
+    for dtype, splits, add in ((torch.float32, 1, False), (torch.float32, 2, False), (torch.bfloat16, 1, False), (torch.float32, 1, True)):
+        size = splits * M * N
+        held = torch.full((size + 512 * N,), 7.0, dtype=dtype, device=DEV)      # what lies behind out
+        out = held[:size].view((splits, M, N) if splits > 1 else (M, N))
+        gemm100.gemm_pair(x, w, out, splits=splits, accumulate=add)
+        gemm100.check_errors(DEV)
+        got = out.double().sum(0) if splits > 1 else out.double()
+        assert rel(got, ref + 7.0 if add else ref) < (3e-5 if dtype == torch.float32 else 5e-3)
+        assert (held[size:] == 7.0).all()
