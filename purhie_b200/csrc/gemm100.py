@@ -88,7 +88,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swapped: bool, 
     out, or plain with block_n 64, 128 or 256): the rows of x lack the factor rsqrt(sum(row_sumsq[m]) / row_width + row_eps);
     the epilogue applies it.  ``norm_ahead`` (weight float32 [N], rows bfloat16 [M, N], sumsq float32 [M, 2 * ceil(N / 256)];
     plain, block_n 256, accumulate): rows = (the new out) * weight, sumsq[m, j] = the sum of squares of the new out
-    over columns 128 j .. 128 j + 127."""
+    over columns 128 j .. 128 j + 127.  The kernel asks for its first tiles of w before the kernel in front of it on the
+    stream has ended: w is a weight, not that kernel's result."""
     for name, t in (("x", x), ("w", w)):
         if not t.is_cuda or t.dtype != torch.bfloat16 or not t.is_contiguous():
             raise KernelError(f"gemm_tcgen05: {name} must be a contiguous bfloat16 CUDA tensor")
