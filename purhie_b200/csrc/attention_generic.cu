@@ -129,6 +129,7 @@ struct F32Params {
 constexpr int RUN_MIN = 4;           // tokens of one request side by side that the tile kernel takes
 constexpr int FEW_ROWS = 9472;       // (token, head) rows below which a warp of the tile kernel takes four instead of eight
 constexpr int LEFT_CTAS = 16;        // CTAs per head for the rows that the tile kernel leaves
+constexpr int FEW_CTAS = 74;         // half of the SMs
 constexpr int KEYS = 128;            // keys a CTA of the rows kernel scores at once
 
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
@@ -201,6 +202,8 @@ __global__ void __launch_bounds__(128, 1) attention_rows_f32_kernel(const F32Par
     long long* at = reinterpret_cast<long long*>(sums + KEYS / 32);   // [2][KEYS] where each key row and value row starts
     const int h = blockIdx.x % p.HQ, g = h / (p.HQ / p.HKV);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     for (int row = blockIdx.x / p.HQ;; row += gridDim.x / p.HQ) {
         // this CTA's next row: of all, or of those that the tile kernel leaves
         const int t = p.tiles ? leftover_token(p.row_seg, p.T, p.tiles, row) : row < p.T ? row : -1;
@@ -542,7 +545,9 @@ int launch_f32(F32Params p, cudaStream_t stream) {
     if (int e = allow_shared<kernel>(bytes, "attention_generic")) return e;
     // (beside tiles few rows are left, most often none: one CTA fits an SM, so a CTA per row that finds nothing to do costs 40 us)
     const int rows = p.tiles && p.T > LEFT_CTAS ? LEFT_CTAS : p.T;
-    kernel<<<(unsigned)((long long)rows * p.HQ), 128, bytes, stream>>>(p);
+    // (started early only where its CTAs are few, as the float32 product)
+    if ((long long)rows * p.HQ <= FEW_CTAS) launch_overlapped(kernel, dim3(rows * p.HQ), dim3(128), bytes, stream, p);
+    else kernel<<<(unsigned)((long long)rows * p.HQ), 128, bytes, stream>>>(p);
     return check_launch("attention_generic");
 }
 

@@ -11,7 +11,8 @@
 //   gemm_rows_f32   float32 with at most 16 rows: the weight streams through a ring in shared memory (decoding)
 //   gemm_tile_f32   float32 with more rows: register tiles, operands by cp.async with k left contiguous
 //   gemm_simple     any other type, K not a multiple of 4 or an operand off 16 bytes
-// The float32 kernels are launched in plain stream order: started early, their CTAs pile up on the SMs that the kernel in
+// The float32 kernels start early only where their CTAs are few (at most one for every second SM:
+// a tiny model's three streams of 12 tokens 1.78 -> 1.64 ms).  Elsewhere, started early, their CTAs pile up on the SMs that the kernel in
 // front leaves first, and with one or two CTAs an SM that imbalance cost a 256-row layer of a 0.6B
 // model 61 us (428 against 367).
 #include "common.cuh"
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(const float* __restr
     static_assert(WORKERS <= 128 && MB % RM == 0, "one CTA holds every output");
     const int tid = threadIdx.x, n0 = blockIdx.x * BN_;
     const int chunks = (K + KC - 1) / KC;
+    pdl_wait();
     auto request = [&](int c) {
         if (c < chunks) {
             float* dst = ring + (size_t)(c % STAGES) * ROWS * KC_STRIDE;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(64) gemm_tile_f32_kernel(const float* __restri
     const int tid = threadIdx.x, lane = tid & 31, tx = lane & 7, ty = tid >> 5 << 2 | lane >> 3;
     const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
     const int chunks = (K + BK32 - 1) / BK32;
+    pdl_wait();
     auto request = [&](int c) {
         if (c < chunks) {
             float* dst = ring + (size_t)(c % TILE_STAGES) * ROWS * BK32_STRIDE;
@@ -265,7 +268,9 @@ int launch_rows(const float* x, const float* w, float* y, int M, int N, int K, c
     const size_t bytes = (size_t)STAGES * (BN_ + MB) * KC_STRIDE * sizeof(float);
     constexpr auto kernel = gemm_rows_f32_kernel<BN_, MB, RM, STAGES>;
     if (int e = allow_shared<kernel>(bytes, "gemm_simple")) return e;
-    kernel<<<(N + BN_ - 1) / BN_, 128, bytes, stream>>>(x, w, y, M, N, K);
+    const int ctas = (N + BN_ - 1) / BN_;
+    if (2 * ctas <= multiprocessors()) launch_overlapped(kernel, dim3(ctas), dim3(128), bytes, stream, x, w, y, M, N, K);
+    else kernel<<<ctas, 128, bytes, stream>>>(x, w, y, M, N, K);
     return check_launch("gemm_simple");
 }
 
@@ -292,7 +297,9 @@ int gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, cuda
     // (16 rows as tiles: 20.5 against 18.9 us at 6144 x 1024, 52 against 17.5 at 1024 x 3072)
     constexpr size_t bytes = (size_t)TILE_STAGES * 2 * TILE * BK32_STRIDE * sizeof(float);
     if (int e = allow_shared<gemm_tile_f32_kernel>(bytes, "gemm_simple")) return e;
-    gemm_tile_f32_kernel<<<dim3((N + TILE - 1) / TILE, (M + TILE - 1) / TILE), 64, bytes, stream>>>(x, w, y, M, N, K);
+    const dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
+    if (2ll * grid.x * grid.y <= multiprocessors()) launch_overlapped(gemm_tile_f32_kernel, grid, dim3(64), bytes, stream, x, w, y, M, N, K);
+    else gemm_tile_f32_kernel<<<grid, 64, bytes, stream>>>(x, w, y, M, N, K);
     return check_launch("gemm_simple");
 }
 
