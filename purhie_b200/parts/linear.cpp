@@ -29,50 +29,75 @@ GemmPlan plan_few(int M, int N, int K, int sms, bool allow_split) {
     return p;
 }
 
-// Many tokens, plain orientation: tiles of 128 tokens x 64, 128 or 256 features on one CTA, or of 256 x 256 on a pair of SMs,
-// and into how many parts K is cut.  Estimated microseconds, fitted to products of 128 to 2,048 tokens with 1,024 to 16,384
-// features and K 1,024 to 8,192: what a launch costs (the pair kernel does not start early), plus rounds of the CTAs times a
-// round's blocks of K, start and epilogue (longer with an activation), plus the float32 partial results' way to memory and
-// back when K is split.  A fused epilogue needs the whole sum in one place.  The narrow tiles are for products whose wide
-// tiles would leave most SMs without one: 256 x 6144 x 1024 with the activation 11.1 us with tiles of 64 columns, 20.1 with
-// 256, 16.0 on pairs; 544 x 1024 x 2048 8.1 us with tiles of 128 and three parts of K, 9.6 on pairs with six; 544 x 4096 x 1024
-// 10.4 us with tiles of 256 on one CTA, 11.6 on pairs.  A long K that stays whole without an activation keeps the wide tiles:
-// by itself 1024 x 2048 x 2048 takes 14.2 us with tiles of 128 and 16.7 on pairs, in a model's chain of launches it was no
-// faster (15 us of 2,060 slower for a prompt of a model of that width).
-void plan_many(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue, GemmPlan& p) {
+// Many tokens, plain orientation: into how many parts K is cut.  A cut K hands float32 sums on where a whole K is written in
+// the output's type (a q or k projection: bfloat16 in front of its norm), and the parts fix the order of the additions, so
+// this rule decides the results' bits and knows nothing of the tiles below, all of which add in the same order.  Its estimate
+// is in units of one block of K on tiles of 256 features: rounds of the CTAs (or pairs) times the item's blocks (0.87 of one on
+// a pair) plus six for start and epilogue, plus the partial results' way to memory and back.  A fused epilogue needs the
+// whole sum in one place.
+int parts_of_k(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue) {
     const int kblocks = ceil_div(K, kBlockK);
     static const int kAll[] = {1, 2, 3, 4, 6, 8};
-    struct Kind { bool pair; int bn, per_sm; double launch, block, item, activation; };
-    static const Kind kKinds[] = {{false, 256, 1, 1.8, 0.31, 5.0, 6.0}, {true, 256, 0, 4.5, 0.28, 3.0, 4.5},
-                                  {false, 128, 1, 1.8, 0.255, 2.2, 4.5}, {false, 64, 2, 1.8, 0.28, 2.0, 0.5}};
     const int n_options = (allow_split && !fused_epilogue) ? 6 : 1;
     double best = -1.0;
-    p.pair = false;
-    p.splits = 1;
-    for (const Kind& k : kKinds) {
-        if (k.pair && (M <= 128 || N <= 128)) continue;
-        const int tiles = ceil_div(M, k.pair ? 256 : 128) * ceil_div(N, k.bn);
-        const int slots = k.pair ? sms / 2 : sms * k.per_sm;
+    int parts = 1;
+    for (int pair = 0; pair < 2; pair++) {
+        if (pair && (M <= 128 || N <= 128)) continue;
+        const int tiles = (pair ? ceil_div(M, 256) : ceil_div(M, 128)) * ceil_div(N, 256);
+        const int slots = pair ? sms / 2 : sms;
         for (int o = 0; o < n_options; o++) {
             const int s = kAll[o];
-            if (s > 1 && (kblocks / s < 8 || k.bn == 64)) continue;
-            if (s == 1 && n_options > 1 && k.bn < 256 && kblocks >= 32) continue;
+            if (s > 1 && kblocks / s < 8) continue;
             const int rounds = ceil_div((long long)tiles * s, slots);
-            double cost = k.launch + rounds * (k.block * kblocks / s + k.item + (fused_epilogue ? k.activation : 0.0));
-            if (s > 1) cost += 2.0 * s * (double)M * N * 4 / 4.0e6;
-            if (best < 0 || cost < best - 1e-9) { best = cost; p.pair = k.pair; p.splits = s; p.block_n = k.bn; }
+            double cost = rounds * ((pair ? 0.87 : 1.0) * kblocks / s + 6.0);
+            if (s > 1) cost += 2.0 * s * (double)M * N * 4 / 4.0e12 / 0.33e-6;
+            if (best < 0 || cost < best - 1e-9) { best = cost; parts = s; }
         }
+    }
+    return parts;
+}
+
+// The tiles for that many parts: 128 tokens x 64, 128 or 256 features on one CTA, or 256 x 256 on a pair of SMs.  Estimated
+// microseconds: a launch (the pair kernel does not start early), rounds of the CTAs times an item's start and epilogue
+// (longer with an activation or the addition into the output), and the longer of the rounds' blocks of K and the tiles' way to
+// the SMs (the weight from memory at 7.3 TB/s, and what every tile reads of both operands from L2 at 22 TB/s).  Fitted to 964
+// launches at 128 to 2,048 tokens, 1,024 to 24,576 features and K 1,024 to 12,288 (root mean square error 9 %); the tiles
+// it picks take 0.3 % longer than the best of the four, summed over those 294 products, 6 % less than tiles of 256 and pairs
+// alone.  Narrow tiles are for products whose wide ones leave most SMs without one: 256 x 6144 x 1024 with the activation
+// 11.3 us with tiles of 64, 16.7 on pairs; 544 x 1024 x 2048 in three parts 8.2 us with tiles of 128, 11.2 on pairs; 544 x 4096 x
+// 1024 10.6 us with tiles of 256 on one CTA, 12.0 on pairs.
+// wide: only tiles of 256 features, whose epilogue also does the work of the norm behind an addition.
+void tiles_for(int M, int N, int K, int sms, bool fused_epilogue, bool adds, bool wide, GemmPlan& p) {
+    const int kblocks = ceil_div(K, kBlockK), s = p.splits;
+    struct Kind { bool pair; int bn, per_sm; double launch, block, item, activation, addition; };
+    static const Kind kKinds[] = {{false, 256, 1, 4.5, 0.307, 3.0, 7.8, 8.5}, {true, 256, 0, 7.4, 0.318, 0.0, 4.0, 2.4},
+                                  {false, 128, 1, 3.9, 0.274, 0.75, 3.8, 2.8}, {false, 64, 2, 3.9, 0.299, 0.0, 0.9, 3.6}};
+    const double weight_mb = 2e-6 * N * K, x_mb = 2e-6 * M * K;
+    double best = -1.0;
+    for (const Kind& k : kKinds) {
+        if (k.pair && (M <= 128 || N <= 128)) continue;
+        if (wide && k.bn < 256) continue;
+        if (s > 1 && k.bn == 64) continue;
+        const int rows = ceil_div(M, k.pair ? 256 : 128), columns = ceil_div(N, k.bn);
+        const int rounds = ceil_div((long long)rows * columns * s, k.pair ? sms / 2 : sms * k.per_sm);
+        const double item = k.item + (fused_epilogue ? k.activation : adds && s == 1 ? k.addition : 0.0);
+        const double cost = k.launch + rounds * item +
+                            std::max(rounds * k.block * kblocks / s, 0.137 * weight_mb + 0.0455 * (rows * weight_mb + columns * x_mb));
+        if (best < 0 || cost < best - 1e-9) { best = cost; p.pair = k.pair; p.block_n = k.bn; }
     }
 }
 }  // namespace
 
-GemmPlan plan_gemm(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue) {
+GemmPlan plan_gemm(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue, bool adds, bool wide) {
     if (M < 128) return plan_few(M, N, K, sms, allow_split);
     GemmPlan p;
     p.swapped = false;
     p.block_n = N > 128 ? 256 : N > 64 ? 128 : 64;
     p.splits = 1;
-    if (p.block_n == 256) plan_many(M, N, K, sms, allow_split, fused_epilogue, p);
+    if (p.block_n == 256) {
+        p.splits = parts_of_k(M, N, K, sms, allow_split, fused_epilogue);
+        tiles_for(M, N, K, sms, fused_epilogue, adds, wide, p);
+    }
     return p;
 }
 
@@ -103,8 +128,8 @@ bool Linear::applies_row_scale(int rows, DType out_dtype, bool fuse_swiglu, bool
     const GemmPlan p = plan_gemm(rows, (int)weight_.shape[0], (int)weight_.shape[1], sm_count(), allow_split, fused);
     // few rows: the fused activation keeps K whole and writes bfloat16 from the swapped epilogue, which is where the factor goes
     if (p.swapped) return out_dtype == DType::BF16 && fused;
-    // many rows: the epilogue of tiles of 64 features and more, whenever it holds whole sums
-    return p.block_n >= 64 && p.splits == 1;
+    // many rows: the epilogue of whatever tiles a weight of more than 128 rows gets, whenever it holds whole sums
+    return weight_.shape[0] > 128 && p.splits == 1;
 }
 
 bool Linear::gives_partial_sums(int rows, bool allow_split) const {
@@ -162,12 +187,10 @@ Addend Linear::operator()(const Tensor& x_in, StepContext& ctx, const std::strin
     }
     const GemmKernels& g = gemm_kernels();
     const bool fused = fuse_swiglu && N % 2 == 0;
-    GemmPlan p = plan_gemm(M, N, K, sm_count(), allow_split, fused);
-    if (add_into && ctx.residual_width == N && ahead && ahead->offered() && !p.swapped && p.splits == 1 && p.block_n < 256 && N > 128) {
-        // the epilogue of wide tiles also does the next norm's work, which saves the norm's launch behind narrow ones
-        p.block_n = 256;
-        p.pair = M > 128;          // 1024 x 2048 x 2048 with the addition: 18.9 us, 23.9 on one CTA
-    }
+    const bool adds = add_into && ctx.residual_width == N;
+    // the norm behind an addition is done in the epilogue wherever K is whole and its rule allows (wide tiles only)
+    const bool norm_ahead = adds && ahead && ahead->offered() && ahead->width == N && N % 4 == 0;
+    const GemmPlan p = plan_gemm(M, N, K, sm_count(), allow_split, fused, adds, norm_ahead);
     auto run = [&](Tensor& out, int splits, bool swiglu, bool accumulate, NormAhead* work_ahead = nullptr) {
         if (LaunchProfile::get().on())      // what the product has to move and to compute: the weight once, x, and its result
             LaunchProfile::get().note_cost(2.0 * N * K + 2.0 * M * K + (double)out.bytes(), 2.0 * M * N * K);
@@ -201,11 +224,10 @@ Addend Linear::operator()(const Tensor& x_in, StepContext& ctx, const std::strin
         run(out, 1, true, false);
         return Addend(out, 1, true);
     }
-    if (add_into && !p.swapped && p.splits == 1 && ctx.residual_width == N) {
+    if (adds && !p.swapped && p.splits == 1) {
         // many tokens, K whole: the residual sum happens in the epilogue and the product never goes to memory
         Tensor target(add_into, DType::F32, {M, N});
-        const bool work_ahead = ahead && ahead->offered() && ahead->width == N && p.block_n == 256 && N % 4 == 0;
-        run(target, 1, false, true, work_ahead ? ahead : nullptr);
+        run(target, 1, false, true, norm_ahead && p.block_n == 256 ? ahead : nullptr);
         return Addend();
     }
     Tensor out = p.splits > 1 ? ws.get(out_name + "_partial", {p.splits, M, N}, DType::F32) : ws.get(out_name, {M, N}, out_dtype);

@@ -18,8 +18,9 @@ struct GemmPlan {
     int splits = 1;          // parts of K, float32 partial sums
     bool pair = false;       // 256 x 256 tiles on pairs of CTAs
 };
-// The shape of the tcgen05 product for M tokens and an [N, K] weight on a device of `sms` SMs.
-QE_API GemmPlan plan_gemm(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue);
+// The shape of the tcgen05 product for M tokens and an [N, K] weight on a device of `sms` SMs.  adds: a whole sum is added into
+// the output; wide: on tiles of 256 features (neither changes the parts of K, nor a result's bits).
+QE_API GemmPlan plan_gemm(int M, int N, int K, int sms, bool allow_split, bool fused_epilogue, bool adds = false, bool wide = false);
 
 class QE_API Linear {
 public:
@@ -50,7 +51,7 @@ public:
     // swapped).  Its partial sums are linear in the rows, and its bfloat16 epilogue can apply a factor per row.
     bool swapped_for(int rows, bool allow_split, bool fused_epilogue) const;
     // The product's own epilogue multiplies by the rows' factor: few rows with the fused activation; many rows
-    // (tiles of 64 features and more) whenever K stays whole and nothing is added into the output.
+    // (a weight of more than 128) whenever K stays whole and nothing is added into the output.
     bool applies_row_scale(int rows, DType out_dtype, bool fuse_swiglu, bool allow_split = true) const;
     // Many rows, K cut into parts: float32 partial sums, linear in the rows, so whoever adds them up can apply the factor.
     bool gives_partial_sums(int rows, bool allow_split) const;
