@@ -24,6 +24,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 namespace {
 
 using namespace ph;
@@ -127,9 +129,7 @@ struct F32Params {
 };
 
 constexpr int RUN_MIN = 4;           // tokens of one request side by side that the tile kernel takes
-constexpr int FEW_ROWS = 9472;       // (token, head) rows below which a warp of the tile kernel takes four instead of eight
-constexpr int LEFT_CTAS = 16;        // CTAs per head for the rows that the tile kernel leaves
-constexpr int FEW_CTAS = 74;         // half of the SMs
+constexpr int FEW_ROWS_PER_SM = 64;  // (token, head) rows an SM below which a warp of the tile kernel takes four instead of eight
 constexpr int KEYS = 128;            // keys a CTA of the rows kernel scores at once
 
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
@@ -158,38 +158,46 @@ __device__ __forceinline__ int ones_from(unsigned mask, int b) {
     const unsigned gap = ~mask >> b;
     return gap ? __ffs(gap) - 1 : 32 - b;
 }
-// The wanted-th (from 0) token, of all in order, that lies in a run shorter than RUN_MIN, runs being cut at multiples of
-// `tile` tokens (8, 16 or 32); -1: there are fewer.  All lanes of a warp call it.
-__device__ int leftover_token(const int32_t* row_seg, int T, int tile, int wanted) {
-    const int lane = threadIdx.x & 31;
-    for (int base = 0; base < T; base += 128) {
-        int seg[4];
+// The tokens, in order, that lie in a run shorter than RUN_MIN, runs being cut at multiples of `tile` tokens (8, 16 or 32).
+struct Leftovers {
+    const int32_t* row_seg;
+    int T, tile;
+    int base = 0, before = 0;                          // the tokens from `base` on have `before` such tokens in front of them
+    // The wanted-th (from 0; no smaller than in the call before) of them; -1: there are fewer.  All lanes of a warp call it.
+    __device__ int token(int wanted) {
+        const int lane = threadIdx.x & 31;
+        for (; base < T; base += 128) {
+            int seg[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = base + 32 * i + lane;
-            seg[i] = t < T ? row_seg[t] : -1;
-        }
+            for (int i = 0; i < 4; ++i) {
+                const int t = base + 32 * i + lane;
+                seg[i] = t < T ? row_seg[t] : -1;
+            }
+            int count = before;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int before = __shfl_up_sync(0xffffffffu, seg[i], 1);
-            const unsigned joined = __ballot_sync(0xffffffffu, lane % tile != 0 && seg[i] == before);      // to the token in front
-            const int start = lane - ones_from(__brev(joined), 31 - lane);
-            const bool left = base + 32 * i + lane < T && 1 + ones_from(joined, start + 1) < RUN_MIN;
-            const unsigned lefts = __ballot_sync(0xffffffffu, left);
-            if (wanted < __popc(lefts)) return base + 32 * i + (int)__fns(lefts, 0, wanted + 1);
-            wanted -= __popc(lefts);
+            for (int i = 0; i < 4; ++i) {
+                const int front = __shfl_up_sync(0xffffffffu, seg[i], 1);
+                const unsigned joined = __ballot_sync(0xffffffffu, lane % tile != 0 && seg[i] == front);      // to the token in front
+                const int start = lane - ones_from(__brev(joined), 31 - lane);
+                const bool left = base + 32 * i + lane < T && 1 + ones_from(joined, start + 1) < RUN_MIN;
+                const unsigned lefts = __ballot_sync(0xffffffffu, left);
+                if (wanted < count + __popc(lefts)) return base + 32 * i + (int)__fns(lefts, 0, wanted - count + 1);
+                count += __popc(lefts);
+            }
+            before = count;
         }
+        return -1;
     }
-    return -1;
-}
+};
 
-// One CTA of 128 threads per (token row, query head), or LEFT_CTAS per head for what the tile kernel leaves.  KEYS keys at a
+// One CTA of 128 threads per (token row, query head), or as many as the device holds for what the tile kernel leaves.  KEYS keys at a
 // time: their rows come by cp.async (the values of a block under its scores, the keys of the next block under the values'
 // sums), thread j scores key j, every warp takes the maximum and the sum of its 32 keys, and thread d adds up output d over
 // the keys in order.  What bounds it: the chain of KEYS dependent multiply-adds of a score's D numbers and of an output's
 // KEYS keys per block, one warp a scheduler.  Four rows of 256 keys, 16 heads of 128: 9.4 us (the plain kernel 214); eight rows of
 // 1,024: 31 us (836).
-template <int D>
+// LEFT: only the rows that the tile kernel leaves (the search costs registers, and with them CTAs an SM at D = 32).
+template <int D, bool LEFT>
 __global__ void __launch_bounds__(128, 1) attention_rows_f32_kernel(const F32Params p) {
     constexpr int KS = D + 4;
     extern __shared__ __align__(16) float smem[];
@@ -204,9 +212,10 @@ __global__ void __launch_bounds__(128, 1) attention_rows_f32_kernel(const F32Par
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
     pdl_wait();
+    Leftovers leftovers{p.row_seg, p.T, p.tiles};
     for (int row = blockIdx.x / p.HQ;; row += gridDim.x / p.HQ) {
         // this CTA's next row: of all, or of those that the tile kernel leaves
-        const int t = p.tiles ? leftover_token(p.row_seg, p.T, p.tiles, row) : row < p.T ? row : -1;
+        const int t = LEFT ? leftovers.token(row) : row < p.T ? row : -1;
         if (t < 0) return;
         const int z = p.positions[t], lo = first_seen(z, p.window, p.chunk);
         const int32_t* table = p.block_table + (size_t)p.row_seg[t] * p.table_stride;
@@ -529,26 +538,42 @@ int launch_tiles_f32(F32Params& p, cudaStream_t stream) {
     return check_launch("attention_generic");
 }
 
+template <int D, bool LEFT>
+int launch_rows_f32(const F32Params& p, cudaStream_t stream) {
+    constexpr size_t bytes = (size_t)(KEYS * (D + 4) + KEYS * D + D + KEYS + 2 * (KEYS / 32)) * sizeof(float) + 2 * KEYS * sizeof(long long);
+    constexpr auto kernel = attention_rows_f32_kernel<D, LEFT>;
+    if (int e = allow_shared<kernel>(bytes, "attention_generic")) return e;
+    long long rows = p.T;
+    if (LEFT) {
+        // How many rows the tiles leave is known on the device only: all of a batch of decoded tokens, none of a prompt.  So as
+        // many CTAs as run at once take them in turn.  512 decoded tokens of 200 keys, 4 heads of 32: 38 us (16 CTAs a head: 212,
+        // the plain kernel 176); 256 portions of three: 35 (249, 105); 64 tokens of 1,024 keys, one head of 128: 44 (138, 1,708);
+        // a prompt of 512, which leaves none, one head of 128: 60 (60).  A CTA per row that finds nothing to do costs 40 us at
+        // 256 rows of 16 heads of 128, one to an SM.
+        static thread_local int per_sm = 0;                            // (a property of the kernel, the same on every device it is built for)
+        if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, bytes) != cudaSuccess || per_sm < 1)) per_sm = 1;
+        rows = std::min<long long>(rows, std::max(1, multiprocessors() * per_sm / p.HQ));
+    }
+    // (started early only where its CTAs are few, as the float32 product; behind the tile kernel, which lets nothing start before
+    // its own CTAs have ended, always)
+    if (LEFT || 2 * rows * p.HQ <= multiprocessors()) launch_overlapped(kernel, dim3((unsigned)(rows * p.HQ)), dim3(128), bytes, stream, p);
+    else kernel<<<(unsigned)(rows * p.HQ), 128, bytes, stream>>>(p);
+    return check_launch("attention_generic");
+}
+
 // Portions of at least RUN_MIN tokens go to the tile kernel in steps of more than 32 rows without a window; the rows kernel
-// takes the rest of such a step and every other step whole.  Four rows a warp while tiles of eight would leave the schedulers
-// with one or two warps each (16 heads of 128: 39 against 63 us at 256 tokens, 76 against 123 at 512; 242 both ways at 1,024).
+// takes the rest of such a step (all of it, where every portion is short) and every other step whole.  Four rows a warp while
+// tiles of eight would leave the schedulers with one or two warps each (16 heads of 128: 39 against 63 us at 256 tokens, 76
+// against 123 at 512; 242 both ways at 1,024).
 template <int D>
 int launch_f32(F32Params p, cudaStream_t stream) {
     if (p.T > 32 && !p.window && !p.chunk) {
-        const bool two = (p.HQ / p.HKV) % 2 == 0, eight = (long long)p.T * p.HQ >= FEW_ROWS;
+        const bool two = (p.HQ / p.HKV) % 2 == 0, eight = (long long)p.T * p.HQ >= (long long)FEW_ROWS_PER_SM * multiprocessors();
         const int e = two ? (eight ? launch_tiles_f32<D, 2, 8>(p, stream) : launch_tiles_f32<D, 2, 4>(p, stream))
                           : (eight ? launch_tiles_f32<D, 1, 8>(p, stream) : launch_tiles_f32<D, 1, 4>(p, stream));
         if (e) return e;
     }
-    constexpr size_t bytes = (size_t)(KEYS * (D + 4) + KEYS * D + D + KEYS + 2 * (KEYS / 32)) * sizeof(float) + 2 * KEYS * sizeof(long long);
-    constexpr auto kernel = attention_rows_f32_kernel<D>;
-    if (int e = allow_shared<kernel>(bytes, "attention_generic")) return e;
-    // (beside tiles few rows are left, most often none: one CTA fits an SM, so a CTA per row that finds nothing to do costs 40 us)
-    const int rows = p.tiles && p.T > LEFT_CTAS ? LEFT_CTAS : p.T;
-    // (started early only where its CTAs are few, as the float32 product)
-    if ((long long)rows * p.HQ <= FEW_CTAS) launch_overlapped(kernel, dim3(rows * p.HQ), dim3(128), bytes, stream, p);
-    else kernel<<<(unsigned)((long long)rows * p.HQ), 128, bytes, stream>>>(p);
-    return check_launch("attention_generic");
+    return p.tiles ? launch_rows_f32<D, true>(p, stream) : launch_rows_f32<D, false>(p, stream);
 }
 
 }  // namespace

@@ -255,14 +255,6 @@ __global__ void __launch_bounds__(64) gemm_tile_f32_kernel(const float* __restri
     }
 }
 
-int multiprocessors() {
-    static thread_local int known_dev = -1, known = 0;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-    if (dev != known_dev && cudaDeviceGetAttribute(&known, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) known_dev = dev;
-    return known > 0 ? known : 148;
-}
-
 template <int BN_, int MB, int RM, int STAGES>
 int launch_rows(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t stream) {
     const size_t bytes = (size_t)STAGES * (BN_ + MB) * KC_STRIDE * sizeof(float);

@@ -18,4 +18,13 @@ inline int allow_shared(size_t bytes, const char* what) {
     return PH_OK;
 }
 
+// Multiprocessors of the current device.
+inline int multiprocessors() {
+    static thread_local int known_dev = -1, known = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev != known_dev && cudaDeviceGetAttribute(&known, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) known_dev = dev;
+    return known > 0 ? known : 148;
+}
+
 }  // namespace ph

@@ -62,6 +62,48 @@ def test_float32_attention_adds_in_the_plain_kernels_order(segs, HQ, HKV, D, pag
     assert torch.equal(outs[0], outs[1])
 
 
+def attend(case, q, HQ, HKV, D, page_size=16):
+    from purhie_b200.csrc import ops
+    out = torch.full((case["T"], HQ * D), float("nan"), device=DEV)
+    ops.attention_generic(q, case["k_base"], case["v_base"], case["page_stride"], page_size, case["table"], case["row_seg"],
+                          case["positions"], out, num_heads=HQ, num_kv_heads=HKV, head_dim=D, window=None, scale=1.0 / math.sqrt(D))
+    return out
+
+
+# more rows than 32, none or few of them in portions long enough for tiles: decoded tokens alone, portions of three, both
+# beside a prompt; more leftover rows than CTAs a head, and searches over several blocks of 128 tokens
+SHORT = [[(200 - i % 7, 1) for i in range(512)], [(100, 3)] * 256, [(90, 70)] + [(60 + i, 1) for i in range(300)] + [(40, 3)] * 31,
+         [(33 + i, 1) for i in range(33)], [(200, 2), (300, 257), (50, 3), (400, 131), (3, 1)]]
+
+
+@pytest.mark.parametrize("segs", SHORT)
+@pytest.mark.parametrize("HQ,HKV,D", [(1, 1, 128), (4, 2, 32), (16, 8, 64)])
+def test_rows_that_tiles_leave_add_in_the_plain_kernels_order(segs, HQ, HKV, D):
+    case = paged_case(segs, HQ, HKV, D, 16, torch.float32, seed=8)
+    out, plain = attend(case, case["q"], HQ, HKV, D), attend(case, off_by_one(case["q"]), HQ, HKV, D)
+    assert not torch.isnan(out).any() and torch.equal(out, plain)
+
+
+@pytest.mark.parametrize("segs", SHORT[:2])
+@pytest.mark.parametrize("HQ,HKV,D", [(2, 2, 64), (4, 2, 32)])
+def test_rows_that_tiles_leave_are_not_slower_than_in_the_plain_kernel(segs, HQ, HKV, D):
+    """Few heads and hundreds of short portions: 16 CTAs a head once took up to 2.4 times the plain kernel's time."""
+    case = paged_case(segs, HQ, HKV, D, 16, torch.float32, seed=8)
+    times = []
+    for q in (case["q"], off_by_one(case["q"])):
+        best = math.inf
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                attend(case, q, HQ, HKV, D)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert times[0] < times[1]
+
+
 @pytest.mark.parametrize("cap", [0.0, 2.0])
 @pytest.mark.parametrize("D", [32, 128])
 def test_float32_attention_with_sink_bias_gate_and_cap(D, cap):
