@@ -18,7 +18,7 @@ from .ops import KernelError, call, register_signatures
 
 register_signatures("gemm100", {
     "ph_gemm_bf16_tcgen05": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                             c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
+                             c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                              c_void_p],
     "ph_gemm_bf16_tcgen05_pair": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                   c_int, c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
@@ -80,16 +80,16 @@ def sm_count(device) -> int:
 
 def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swapped: bool, block_n: int, splits: int = 1,
          max_ctas: int = 0, swiglu: bool = False, accumulate: bool = False, row_sumsq: Optional[torch.Tensor] = None, gate=None,
-         row_width: int = 0, row_eps: float = 0.0, norm_ahead: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = None
-         ) -> torch.Tensor:
+         row_width: int = 0, row_eps: float = 0.0, norm_ahead: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = None,
+         early_w: bool = False) -> torch.Tensor:
     """out[M, N] = x[M, K] @ w[N, K]^T (out [splits, M, N] float32 partial sums when splits > 1).  With
     ``swiglu`` the rows of w are (gate, up) pairs and out is [M, N / 2] = silu(gate) * up.  ``accumulate``
     (plain orientation, float32, one split): out += the product.  ``row_sumsq`` [M, chunks] (swapped with bfloat16
     out, or plain with block_n 64, 128 or 256): the rows of x lack the factor rsqrt(sum(row_sumsq[m]) / row_width + row_eps);
     the epilogue applies it.  ``norm_ahead`` (weight float32 [N], rows bfloat16 [M, N], sumsq float32 [M, 2 * ceil(N / 256)];
     plain, block_n 256, accumulate): rows = (the new out) * weight, sumsq[m, j] = the sum of squares of the new out
-    over columns 128 j .. 128 j + 127.  The kernel asks for its first tiles of w before the kernel in front of it on the
-    stream has ended: w is a weight, not that kernel's result."""
+    over columns 128 j .. 128 j + 127.  ``early_w`` (plain; swapped always): the first tiles of w may be read before the kernel
+    in front on the stream has ended, so w is a weight, not that kernel's result."""
     for name, t in (("x", x), ("w", w)):
         if not t.is_cuda or t.dtype != torch.bfloat16 or not t.is_contiguous():
             raise KernelError(f"gemm_tcgen05: {name} must be a contiguous bfloat16 CUDA tensor")
@@ -100,7 +100,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swapped: bool, 
     call("gemm100", "ph_gemm_bf16_tcgen05", x.data_ptr(), w.data_ptr(), out.data_ptr(), ops._code(out.dtype), M, N, K,
          1 if swapped else 0, block_n, splits, max_ctas, 1 if swiglu else 0, _gate_pointer(gate), 1 if accumulate else 0,
          None if row_sumsq is None else row_sumsq.data_ptr(), 0 if row_sumsq is None else row_sumsq.shape[-1], row_width,
-         float(row_eps), *_norm_ahead_pointers(norm_ahead, M, N), error_flag(x.device).data_ptr(), ops._stream())
+         float(row_eps), *_norm_ahead_pointers(norm_ahead, M, N), 1 if early_w else 0, error_flag(x.device).data_ptr(), ops._stream())
     return out
 
 

@@ -80,6 +80,9 @@ struct GemmParams {
     // null) multiplies the rows of the accumulator in front of the activation.
     const int32_t* tile_group;
     const float* row_factor;
+    // One-CTA kernel: the weight was complete before the kernel in front of this one started, so its first tiles are asked for
+    // before that kernel has ended.
+    int early_w;
     int* error_flag;
 };
 
@@ -534,7 +537,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             wb.start(blockIdx.x, work_total);
             int pre = 0;
             // fill the (still empty) ring with tiles of the weight now: A in the swapped orientation, B in the plain one
-            for (; pre < STAGES && wa.valid; ++pre) {
+            for (; p.early_w && pre < STAGES && wa.valid; ++pre) {
                 mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
                 if (p.swapped) tma_load_2d(smem_a + pre * A_BYTES, &map_a, &full[pre], wa.kb * BK, wa.a0);
                 else tma_load_2d(smem_b + pre * Cfg::B_BYTES, &map_b, &full[pre], wa.kb * BK, wa.b0);
@@ -1205,7 +1208,7 @@ PH_EXPORT int ph_gemm_bf16_tcgen05_pair(const void* x, const void* w, void* out,
     p.rows_a = M; p.rows_b = N; p.K = K;
     p.a_tiles = 0; p.b_tiles = (N + PAIR_BN - 1) / PAIR_BN; p.splits = splits; p.kblocks = kblocks;
     p.out = out; p.out_bf16 = out_dtype == PH_BF16; p.swapped = 0; p.swiglu = swiglu; p.gate_kind = gate ? (int)gate[3] : 0; p.gate_alpha = gate ? gate[0] : 1.0f; p.gate_limit = gate ? gate[1] : 0.0f; p.gate_shift = gate ? gate[2] : 0.0f; p.accumulate = accumulate; p.ld = swiglu ? N / 2 : N;
-    p.split_stride = (long long)M * N; p.error_flag = error_flag; p.tile_group = nullptr; p.row_factor = nullptr;
+    p.split_stride = (long long)M * N; p.error_flag = error_flag; p.tile_group = nullptr; p.row_factor = nullptr; p.early_w = 0;
     p.row_sumsq = row_sumsq; p.row_chunks = row_chunks; p.row_width = row_width; p.row_eps = row_eps;
     p.norm_weight = norm_weight; p.norm_rows = (__nv_bfloat16*)norm_rows; p.norm_sumsq = norm_sumsq;
     // bfloat16 results of whole sums leave through the copy engine where its rules allow (rows of a multiple of 16 bytes)
@@ -1256,10 +1259,12 @@ PH_EXPORT int ph_gemm_bf16_tcgen05_grouped(const void* x, const void* w, void* o
 // row_sumsq [M][row_chunks] (or null), row_width, row_eps: the activations lack a factor per token, see GemmParams;
 // taken by the swapped orientation with bfloat16 output, and by the plain orientation with tiles of 256 columns.
 // norm_weight, norm_rows, norm_sumsq: as in the pair kernel (plain orientation, block_n 256, accumulate).
+// early_w: w is not a result of the kernel in front on the stream, nor of one that may still run then, and its first tiles may
+// be read before that kernel has ended.  The swapped orientation always does that: its w has to be such a weight.
 PH_EXPORT int ph_gemm_bf16_tcgen05(const void* x, const void* w, void* out, int out_dtype, int M, int N, int K,
                                    int swapped, int block_n, int splits, int max_ctas, int swiglu, const float* gate, int accumulate,
                                    const float* row_sumsq, int row_chunks, int row_width, float row_eps,
-                                   const float* norm_weight, void* norm_rows, float* norm_sumsq,
+                                   const float* norm_weight, void* norm_rows, float* norm_sumsq, int early_w,
                                    int* error_flag, cudaStream_t stream) {
     if (!x || !w || !out || !error_flag || M < 1 || N < 1 || K < 1 || !valid_dtype(out_dtype))
         return fail(PH_ERR_ARG, "gemm_tcgen05: bad arguments (M %d, N %d, K %d)", M, N, K);
@@ -1300,6 +1305,7 @@ PH_EXPORT int ph_gemm_bf16_tcgen05(const void* x, const void* w, void* out, int 
     p.row_sumsq = row_sumsq; p.row_chunks = row_chunks; p.row_width = row_width; p.row_eps = row_eps;
     p.norm_weight = norm_weight; p.norm_rows = (__nv_bfloat16*)norm_rows; p.norm_sumsq = norm_sumsq;
     p.tma_store = 0;
+    p.early_w = swapped || early_w;
     const bool scaled = !swapped && row_sumsq != nullptr;
     switch (block_n) {
         case 16: return launch<16, false>(ma, mb, p, max_ctas, stream);

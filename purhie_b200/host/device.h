@@ -267,7 +267,7 @@ struct LatentKernels {
 };
 struct GemmKernels {
     int (*gemm)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const float*, int, const float*, int, int,
-                float, const float*, void*, float*, int*, cudaStream_t);
+                float, const float*, void*, float*, int, int*, cudaStream_t);
     int (*gemm_pair)(const void*, const void*, void*, int, int, int, int, int, int, int, const float*, int, const float*, int, int, float,
                      const float*, void*, float*, int*, cudaStream_t);
     // several weights in one launch, a weight per tile of 256 rows

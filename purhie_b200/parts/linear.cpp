@@ -153,14 +153,14 @@ void Linear::into(const Tensor& x_in, StepContext& ctx, Tensor out, int rows) co
         QE_LAUNCH(core, core.gemm_simple(x.data, x.code(), weight_.data, weight_.code(), out.data, out.code(), M, N, K, ctx.stream));
         return;
     }
-    const GemmKernels& g = gemm_kernels();
+    const GemmKernels& g = gemm_kernels();      // (weights are complete before the first step: their tiles are asked for early)
     const GemmPlan p = plan_gemm(M, N, K, sm_count(), false, false);
     if (p.pair)
         QE_LAUNCH(g, g.gemm_pair(x.data, weight_.data, out.data, out.code(), M, N, K, 1, 0, 0, nullptr, 0, nullptr, 0, 0, 0.0f, nullptr,
                                  nullptr, nullptr, ctx.gemm_error, ctx.stream));
     else
         QE_LAUNCH(g, g.gemm(x.data, weight_.data, out.data, out.code(), M, N, K, p.swapped, p.block_n, 1, 0, 0, nullptr, 0, nullptr, 0, 0,
-                            0.0f, nullptr, nullptr, nullptr, ctx.gemm_error, ctx.stream));
+                            0.0f, nullptr, nullptr, nullptr, 1, ctx.gemm_error, ctx.stream));
 }
 
 Addend Linear::operator()(const Tensor& x_in, StepContext& ctx, const std::string& out_name, DType out_dtype, int rows,
@@ -214,7 +214,7 @@ Addend Linear::operator()(const Tensor& x_in, StepContext& ctx, const std::strin
                                      width, eps, ahead_weight, ahead_rows, ahead_sumsq, ctx.gemm_error, ctx.stream));
         else
             QE_LAUNCH(g, g.gemm(x.data, weight_.data, out.data, out.code(), M, N, K, p.swapped, p.block_n, splits, 0, swiglu, gate,
-                                accumulate, sumsq, chunks, width, eps, ahead_weight, ahead_rows, ahead_sumsq, ctx.gemm_error,
+                                accumulate, sumsq, chunks, width, eps, ahead_weight, ahead_rows, ahead_sumsq, 1, ctx.gemm_error,
                                 ctx.stream));
     };
     if (fused && (p.swapped || p.splits == 1)) {

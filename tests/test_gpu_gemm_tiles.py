@@ -115,3 +115,25 @@ def test_whole_sums_have_the_same_bits_on_all_tiles(M, N, K, swiglu):
         gemm100.check_errors(DEV)
         outs.append(out)
     assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 200, 64), (517, 1024, 520), (2048, 2304, 1024)])
+@pytest.mark.parametrize("block_n", [64, 128, 256])
+def test_a_weight_that_the_kernel_in_front_makes(M, N, K, block_n):
+    """A plain product is complete when its w is the result of the kernel in front, which lets its dependents start early."""
+    from purhie_b200.csrc import gemm100
+    a, b, x = (rnd(r, c, dtype=torch.bfloat16, seed=s, scale=0.1) for r, c, s in ((N, 4096, 61), (K, 4096, 62), (M, K, 63)))
+    w, out = torch.empty(N, K, dtype=torch.bfloat16, device=DEV), torch.empty(M, N, device=DEV)
+    gemm100.gemm(a, b, w, swapped=False, block_n=256)
+    torch.cuda.synchronize()
+    ref = x.double() @ w.double().T
+    for _ in range(4):
+        w.fill_(float("nan"))
+        out.fill_(float("nan"))
+        gemm100.gemm(a, b, w, swapped=False, block_n=256)
+        gemm100.gemm(x, w, out, swapped=False, block_n=block_n)
+        gemm100.check_errors(DEV)
+        assert rel(out, ref) < 3e-5
+    early = torch.empty_like(out)
+    gemm100.gemm(x, w, early, swapped=False, block_n=block_n, early_w=True)     # (w is complete by now)
+    assert torch.equal(early, out)
