@@ -190,13 +190,13 @@ struct Leftovers {
     }
 };
 
-// One CTA of 128 threads per (token row, query head), or as many as the device holds for what the tile kernel leaves.  KEYS keys at a
+// One CTA of 128 threads per (token row, query head), or one for every SM for what the tile kernel leaves.  KEYS keys at a
 // time: their rows come by cp.async (the values of a block under its scores, the keys of the next block under the values'
 // sums), thread j scores key j, every warp takes the maximum and the sum of its 32 keys, and thread d adds up output d over
 // the keys in order.  What bounds it: the chain of KEYS dependent multiply-adds of a score's D numbers and of an output's
 // KEYS keys per block, one warp a scheduler.  Four rows of 256 keys, 16 heads of 128: 9.4 us (the plain kernel 214); eight rows of
 // 1,024: 31 us (836).
-// LEFT: only the rows that the tile kernel leaves (the search costs registers, and with them CTAs an SM at D = 32).
+// LEFT: only the rows that the tile kernel leaves (the search costs registers, and with them a tenth of the speed at D = 32).
 template <int D, bool LEFT>
 __global__ void __launch_bounds__(128, 1) attention_rows_f32_kernel(const F32Params p) {
     constexpr int KS = D + 4;
@@ -545,14 +545,13 @@ int launch_rows_f32(const F32Params& p, cudaStream_t stream) {
     if (int e = allow_shared<kernel>(bytes, "attention_generic")) return e;
     long long rows = p.T;
     if (LEFT) {
-        // How many rows the tiles leave is known on the device only: all of a batch of decoded tokens, none of a prompt.  So as
-        // many CTAs as run at once take them in turn.  512 decoded tokens of 200 keys, 4 heads of 32: 38 us (16 CTAs a head: 212,
-        // the plain kernel 176); 256 portions of three: 35 (249, 105); 64 tokens of 1,024 keys, one head of 128: 44 (138, 1,708);
-        // a prompt of 512, which leaves none, one head of 128: 60 (60).  A CTA per row that finds nothing to do costs 40 us at
-        // 256 rows of 16 heads of 128, one to an SM.
-        static thread_local int per_sm = 0;                            // (a property of the kernel, the same on every device it is built for)
-        if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, bytes) != cudaSuccess || per_sm < 1)) per_sm = 1;
-        rows = std::min<long long>(rows, std::max(1, multiprocessors() * per_sm / p.HQ));
+        // How many rows the tiles leave is known on the device only: all of a batch of decoded tokens, none of a prompt.  So a CTA for
+        // every SM takes them in turn.  512 decoded tokens of 200 keys, 4 heads of 32: 87 us (with 16 CTAs a head 214, the plain
+        // kernel 176); 256 portions of three: 83 (249, 105); 64 tokens of 1,024 keys, one head of 128: 44 (140, 1,708); a prompt of
+        // 512, which leaves none, one head of 128: 62 (62).  As many CTAs as an SM holds (five at D = 32) would take 38 us for the
+        // first of these, but where nothing is left, as behind a prompt, the kernel behind them then stood still for 13 us (a tiny
+        // model's prompt of 97 tokens and two answers: 381 -> 409 us).
+        rows = std::min<long long>(rows, std::max(1, multiprocessors() / p.HQ));
     }
     // (started early only where its CTAs are few, as the float32 product; behind the tile kernel, which lets nothing start before
     // its own CTAs have ended, always)
