@@ -60,8 +60,7 @@ Engine::Engine(std::shared_ptr<DecoderModel> model, const EngineOptions& options
 
 Engine::~Engine() {
     if (stream_) cudaStreamSynchronize(stream_);
-    for (auto& g : graphs_)
-        if (g.second->exec) cudaGraphExecDestroy(g.second->exec);
+    graphs_.clear();
     for (auto& s : pending_)
         if (s.p.event) cudaEventDestroy(s.p.event);
     for (int i = 0; i < 2; i++)
@@ -386,10 +385,10 @@ Tensor Engine::step_any(const std::vector<StepEntry>& entries, Layout& lay) {
 
 // A batch of single tokens: the launches of the whole model are captured once per (batch size, block table
 // widths, context bucket, what the parts added) and replayed.  Each graph owns its scratch memory and metadata
-// buffer, so nothing it points at ever moves.  The graph of a step that wants logits computes every row's; the wanted
-// ones are picked afterwards.  A step that wants none has a graph of its own, which ends behind the last layer: reading the
-// output matrix takes 0.2 ms at the 8B shape (eight layers, one row, eight steps of which one wants logits: 7.47 -> 6.08 ms)
-// and 0.06 ms at the 0.6B shape (28 layers: 9.25 -> 8.82 ms).
+// buffer, so nothing it points at ever moves.  A step that wants logits computes every row's; the wanted ones are picked
+// afterwards.  A step that wants none (tokens that are given, not sampled) replays a second form of the same graph, in the same
+// memory, which ends behind the last layer: reading the output matrix takes 0.2 ms at the 8B shape (eight layers, one row,
+// eight steps of which one wants logits: 7.47 -> 6.08 ms) and 0.06 ms at the 0.6B shape (28 layers: 9.25 -> 8.82 ms).
 Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* device_tokens, Layout& lay) {
     const int S = (int)entries.size();
     int need = 1;
@@ -397,9 +396,9 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
         for (const PageGroup& g : cache_->groups()) need = std::max(need, (int)cache_->block_table(e.request, g.index).size() + 1);
     bool any_wanted = false;
     for (const StepEntry& e : entries) any_wanted |= e.n_want > 0;
-    layout(entries, pow2_at_least(need, 8), any_wanted, lay);
+    layout(entries, pow2_at_least(need, 8), true, lay);
     const int ctx_bucket = pow2_at_least(lay.decode_max_ctx, 256);
-    std::string key = std::to_string(S) + "|" + std::to_string(ctx_bucket) + (any_wanted ? "|logits" : "");
+    std::string key = std::to_string(S) + "|" + std::to_string(ctx_bucket);
     for (int w : lay.widths) key += "|w" + std::to_string(w);
     for (const auto& a : lay.extra) key += "|" + a.first + ":" + std::to_string(a.second.second);
     Graph* g = nullptr;
@@ -413,7 +412,6 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
         if (!g) {
             if ((int)graphs_.size() >= options_.max_graphs) {
                 QE_CUDA(cudaStreamSynchronize(stream_));
-                if (graphs_.front().second->exec) cudaGraphExecDestroy(graphs_.front().second->exec);
                 graphs_.pop_front();
             }
             std::unique_ptr<Graph> fresh(new Graph());
@@ -427,15 +425,24 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
         upload(lay, g->meta.data());
         if (device_tokens)                                           // the token ids lead the metadata
             QE_CUDA(cudaMemcpyAsync(g->meta.data(), device_tokens, (size_t)S * 4, cudaMemcpyDeviceToDevice, stream_));
-        if (!g->exec) {
+        Graph::Form& form = g->forms[any_wanted];
+        if (!form.exec) {
             StepContext ctx;
             const int32_t* rows = nullptr;
             context(lay, static_cast<const int32_t*>(g->meta.data()), g->workspace, ctx, &rows);
             ctx.decode_max_ctx = ctx_bucket;                         // the number of attention splits must not change between replays
             // the first time: run the launches directly (this is the step's result, and whatever a kernel sets up
             // on first use is set up), then capture the same launches for the next time
-            g->logits = forward(ctx, rows, any_wanted ? S : 0);
+            const long long moves = g->workspace.moves();
+            g->workspace.frozen = false;
+            Tensor logits = forward(ctx, rows, any_wanted ? S : 0);
             g->workspace.frozen = true;
+            if (any_wanted) g->logits = logits;
+            Graph::Form& other = g->forms[!any_wanted];
+            if (g->workspace.moves() != moves && other.exec) {        // scratch memory that the other form points at is gone
+                cudaGraphExecDestroy(other.exec);
+                other.exec = nullptr;
+            }
             const long long before = g_launches;
             QE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeRelaxed));
             cudaGraph_t graph = nullptr;
@@ -447,21 +454,24 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
                 throw;
             }
             QE_CUDA(cudaStreamEndCapture(stream_, &graph));
-            g->launches = g_launches - before;
+            form.launches = g_launches - before;
             g_launches = before;
-            cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
+            cudaError_t e = cudaGraphInstantiate(&form.exec, graph, 0);
             cudaGraphDestroy(graph);
-            if (e != cudaSuccess) { g->exec = nullptr; throw KernelError(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)); }
+            if (e != cudaSuccess) { form.exec = nullptr; throw KernelError(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)); }
             stats_.replayed_graph = false;
         } else {
-            QE_CUDA(cudaGraphLaunch(g->exec, stream_));
-            g_launches += g->launches;
+            QE_CUDA(cudaGraphLaunch(form.exec, stream_));
+            g_launches += form.launches;
             stats_.replayed_graph = true;
             graph_replays_++;
         }
     } catch (...) {
         for (const StepEntry& e : entries) cache_->unreserve(e.request);
-        if (g && !g->exec) graphs_.pop_back();                        // a graph that was never finished is not kept
+        if (g && !g->forms[any_wanted].exec) {                        // a form that was not finished may have moved the other's memory
+            cudaStreamSynchronize(stream_);
+            graphs_.pop_back();
+        }
         throw;
     }
     if (!any_wanted) return Tensor();

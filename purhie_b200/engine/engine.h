@@ -167,13 +167,18 @@ public:
 
 private:
     using Layout = StepLayout;
+    // The launches of a decode step in two forms: behind the last layer, or with the output matrix.  Both work in the same
+    // scratch memory and metadata, one after the other on the engine's stream.
     struct Graph {
+        struct Form {
+            cudaGraphExec_t exec = nullptr;
+            long long launches = 0;
+        };
         Workspace workspace;
         DeviceBuffer meta;
-        cudaGraphExec_t exec = nullptr;
+        Form forms[2];                   // [1]: with the output matrix
         Tensor logits;
-        long long launches = 0;
-        std::string signature;
+        ~Graph() { for (Form& f : forms) if (f.exec) cudaGraphExecDestroy(f.exec); }
     };
     void validate(const std::vector<StepEntry>& entries) const;
     void layout(const std::vector<StepEntry>& entries, int table_width, bool all_rows_wanted, Layout& lay);

@@ -69,6 +69,7 @@ Tensor Workspace::get(const std::string& name, std::vector<int64_t> shape, DType
         if (it != bufs_.end()) {
             QE_CUDA(cudaStreamSynchronize(stream));        // a kernel in flight may still use the old block
             bufs_.erase(it);
+            moves_++;
         }
         it = bufs_.emplace(name, DeviceBuffer(need)).first;
     }

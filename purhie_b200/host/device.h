@@ -79,10 +79,12 @@ public:
     Workspace() = default;
     Tensor get(const std::string& name, std::vector<int64_t> shape, DType dtype);
     size_t bytes() const;
+    long long moves() const { return moves_; }     // how often a name's tensor has moved to a larger block
     bool frozen = false;
     cudaStream_t stream = nullptr;      // growing waits for this stream before the old block is freed
 private:
     std::map<std::string, DeviceBuffer> bufs_;
+    long long moves_ = 0;
 };
 
 // ---- kernel libraries ---------------------------------------------------------------------------------------

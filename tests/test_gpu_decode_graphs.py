@@ -54,3 +54,29 @@ def test_results_that_are_kept_stay_as_they_are():
     for a, b in zip(held, copies):
         assert np.array_equal(a, b)
     assert len({a.ctypes.data for a in held}) == len(held)
+
+
+def test_steps_with_and_without_logits_share_a_place_among_the_graphs():
+    """Two batch sizes in two places: steps of either size, with wanted logits and without, are all replayed in the end, with the
+    logits of an engine that has room for many."""
+    from purhie_b200.engine import Engine, StepEntry
+    toks = [random_tokens(60, TINY_C["vocab_size"], 5 + r) for r in range(2)]
+    results = []
+    for most in (2, 24):
+        eng = Engine.from_random(TINY_C, 3, dtype="bfloat16", page_size=16, max_tokens=1024, max_requests=2, engine_options={"max_graphs": most})
+        for r in range(2):
+            eng.add_request(r)
+            eng.step([StepEntry(r, toks[r][:9], [])])
+        at, kept = [9, 9], []
+        for k in range(24):
+            rows = [0, 1] if k // 2 % 2 else [k // 4 % 2]
+            out = eng.step([StepEntry(r, [toks[r][at[r]]], [0] if k % 2 else []) for r in rows])
+            for r in rows:
+                at[r] += 1
+            assert k < 4 or eng.last_stats.replayed_graph
+            if k % 2:
+                kept.append(out)
+        assert eng.info()["graphs"] == 2
+        eng.close()
+        results.append(np.concatenate(kept))
+    assert np.array_equal(results[0], results[1])
