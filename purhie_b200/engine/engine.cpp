@@ -540,9 +540,8 @@ RowPool::Block* RowPool::take(const std::shared_ptr<RowPool>& pool, size_t bytes
                 pool->free_.erase(pool->free_.begin());
             }
             if (pool->held_ + bytes > kMost) return nullptr;
-            block.reset(new Block());
             try {
-                block->memory.ensure(bytes);
+                block.reset(new Block(bytes));
             } catch (const Error&) {                                             // no page-locked memory left: ordinary memory serves
                 cudaGetLastError();
                 return nullptr;
@@ -556,6 +555,7 @@ RowPool::Block* RowPool::take(const std::shared_ptr<RowPool>& pool, size_t bytes
 
 void RowPool::give(Block* given) {
     std::unique_ptr<Block> block(given);
+    if (!block->memory.own()) return;                                            // (in a forked process: its own copy goes)
     const std::shared_ptr<RowPool> pool = std::move(block->pool);
     std::lock_guard<std::mutex> lock(pool->mutex_);
     pool->free_.push_back(std::move(block));

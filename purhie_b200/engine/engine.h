@@ -90,11 +90,13 @@ QE_API void context_from_layout(const StepLayout& lay, const CacheManager& cache
 // Page-locked memory for results that a caller keeps: a block is taken for one result and given back when the result is
 // gone; blocks are reused.  Copies of several rows of logits into ordinary memory fresh from the allocator took 0.9 to 1.3 ms
 // for 4.9 MB (page faults and the driver's staging), into these blocks 0.1 ms.  At most kMost bytes are held, in use or
-// not; beyond that take() gives nothing and the caller uses ordinary memory.  Safe from any thread.
+// not; beyond that take() gives nothing and the caller uses ordinary memory.  Safe from any thread; a process forked by the
+// caller keeps its own copy of a result and leaves the pool alone.
 class QE_API RowPool {
 public:
     struct Block {
-        PinnedBuffer memory;
+        explicit Block(size_t bytes) : memory(bytes) {}
+        PrivatePinnedBuffer memory;
         std::shared_ptr<RowPool> pool;       // while taken: the pool outlives its engine until the last block is back
     };
     static constexpr size_t kMost = (size_t)64 << 20;

@@ -1,6 +1,8 @@
 #include "device.h"
 
 #include <dlfcn.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <mutex>
 
@@ -44,6 +46,21 @@ void PinnedBuffer::ensure(size_t bytes) {
     QE_CUDA(cudaMallocHost(&p_, bytes));
     n_ = bytes;
 }
+
+PrivatePinnedBuffer::PrivatePinnedBuffer(size_t bytes) : n_(bytes), pid_((int)getpid()) {
+    p_ = mmap(nullptr, n_, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p_ == MAP_FAILED) throw KernelError("no host memory for " + std::to_string(bytes) + " bytes");
+    const cudaError_t e = cudaHostRegister(p_, n_, cudaHostRegisterPortable);
+    if (e != cudaSuccess) {
+        munmap(p_, n_);
+        throw KernelError(std::string("cudaHostRegister: ") + cudaGetErrorString(e));
+    }
+}
+PrivatePinnedBuffer::~PrivatePinnedBuffer() {
+    if (own()) cudaHostUnregister(p_);
+    munmap(p_, n_);
+}
+bool PrivatePinnedBuffer::own() const { return pid_ == (int)getpid(); }
 
 Tensor DeviceArena::alloc(DType dtype, std::vector<int64_t> shape) {
     Tensor t(nullptr, dtype, std::move(shape));

@@ -60,6 +60,24 @@ private:
     size_t n_ = 0;
 };
 
+// Page-locked memory that a program may keep and hand to processes it forks: private pages, of which a child has its own copy,
+// where cudaMallocHost gives pages that parent and child share (a result kept in a child changed under the parent's next steps).
+// The device copies to it as fast (8 MiB: 153 us both).
+class QE_API PrivatePinnedBuffer {
+public:
+    explicit PrivatePinnedBuffer(size_t bytes);      // throws KernelError when there is none to be had
+    ~PrivatePinnedBuffer();
+    PrivatePinnedBuffer(const PrivatePinnedBuffer&) = delete;
+    PrivatePinnedBuffer& operator=(const PrivatePinnedBuffer&) = delete;
+    void* data() const { return p_; }
+    size_t bytes() const { return n_; }
+    bool own() const;                                // false in a process forked since, where it is ordinary memory
+private:
+    void* p_ = nullptr;
+    size_t n_ = 0;
+    int pid_ = 0;
+};
+
 // Device tensors that somebody keeps for good (weights and what parts derive from them).
 class QE_API DeviceArena {
 public:

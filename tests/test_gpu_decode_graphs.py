@@ -80,3 +80,44 @@ def test_steps_with_and_without_logits_share_a_place_among_the_graphs():
         eng.close()
         results.append(np.concatenate(kept))
     assert np.array_equal(results[0], results[1])
+
+
+def test_a_forked_process_keeps_the_results_it_was_given():
+    """Several rows of logits in the pool's memory: what a forked process holds stays as it was while the parent drops its own
+    reference and its next steps use the memory again, and the parent's results are its own."""
+    import os
+    import signal
+    from purhie_b200.engine import Engine, StepEntry
+    config = dict(TINY_C, vocab_size=400000, tie_word_embeddings=True)
+    eng = Engine.from_random(config, 3, dtype="bfloat16", page_size=16, max_tokens=2048, max_requests=2)
+    eng.add_request("a")
+    toks = random_tokens(32, config["vocab_size"], 5)
+    out = eng.step([StepEntry("a", toks[:8], range(8))])
+    expected, block = out.copy(), out.ctypes.data
+    read_end, write_end = os.pipe()
+    child = os.fork()
+    if child == 0:                                        # nothing here but memory and os calls
+        status = 2
+        try:
+            signal.alarm(60)
+            os.read(read_end, 1)
+            status = 0 if np.array_equal(out, expected) else 1
+            del out
+        finally:
+            os._exit(status)
+    del out
+    out = eng.step([StepEntry("a", toks[8:16], range(8))])
+    again, taken = out.copy(), out.ctypes.data
+    os.write(write_end, b"x")
+    status = os.waitstatus_to_exitcode(os.waitpid(child, 0)[1])
+    os.close(read_end)
+    os.close(write_end)
+    assert taken == block                                 # (the memory was indeed used again)
+    assert status == 0
+    assert np.array_equal(out, again) and not np.array_equal(out, expected)
+    eng.close()
+    fresh = Engine.from_random(config, 3, dtype="bfloat16", page_size=16, max_tokens=2048, max_requests=2)
+    fresh.add_request("a")
+    fresh.step([StepEntry("a", toks[:8], [])])
+    assert np.array_equal(fresh.step([StepEntry("a", toks[8:16], range(8))]), again)
+    fresh.close()
