@@ -416,6 +416,12 @@ API void qe_rows_give(void* block) {
         return 0;
     });
 }
+// Bytes of page-locked memory the engine's results hold, in use or not.
+API long long qe_rows_held(inference_model_t* m) {
+    long long held = -1;
+    guarded([&] { held = (long long)need_engine(m).row_pool()->held(); return 0; });
+    return held;
+}
 API long long qe_launches(void) { return g_launches; }
 API void qe_set_library_dir(const char* dir) { set_library_dir(dir ? dir : ""); }
 

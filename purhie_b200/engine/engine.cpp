@@ -531,15 +531,25 @@ RowPool::Block* RowPool::take(const std::shared_ptr<RowPool>& pool, size_t bytes
             const size_t n = pool->free_[i]->memory.bytes();
             if (n >= bytes && n / 2 <= bytes && (best == pool->free_.size() || n < pool->free_[best]->memory.bytes())) best = i;
         }
+        const size_t missed = pool->missed_;
+        pool->missed_ = 0;
         if (best < pool->free_.size()) {
             block = std::move(pool->free_[best]);
             pool->free_.erase(pool->free_.begin() + best);
         } else {
-            while (pool->held_ + bytes > kMost && !pool->free_.empty()) {        // blocks of other sizes make room
+            if (pool->held_ + bytes > kMost) {
+                size_t idle = 0;
+                for (const auto& b : pool->free_) idle += b->memory.bytes();
+                if (bytes > kMost || pool->held_ - idle + bytes > kMost) return nullptr;
+                if (missed < bytes / 2 || missed / 2 > bytes) {
+                    pool->missed_ = bytes;
+                    return nullptr;
+                }
+            }
+            while (pool->held_ + bytes > kMost) {                                // blocks of other sizes make room
                 pool->held_ -= pool->free_.front()->memory.bytes();
                 pool->free_.erase(pool->free_.begin());
             }
-            if (pool->held_ + bytes > kMost) return nullptr;
             try {
                 block.reset(new Block(bytes));
             } catch (const Error&) {                                             // no page-locked memory left: ordinary memory serves
@@ -551,6 +561,11 @@ RowPool::Block* RowPool::take(const std::shared_ptr<RowPool>& pool, size_t bytes
     }
     block->pool = pool;
     return block.release();
+}
+
+size_t RowPool::held() {
+    std::lock_guard<std::mutex> lock(mutex_);
+    return held_;
 }
 
 void RowPool::give(Block* given) {

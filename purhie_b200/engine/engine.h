@@ -90,7 +90,9 @@ QE_API void context_from_layout(const StepLayout& lay, const CacheManager& cache
 // Page-locked memory for results that a caller keeps: a block is taken for one result and given back when the result is
 // gone; blocks are reused.  Copies of several rows of logits into ordinary memory fresh from the allocator took 0.9 to 1.3 ms
 // for 4.9 MB (page faults and the driver's staging), into these blocks 0.1 ms.  At most kMost bytes are held, in use or
-// not; beyond that take() gives nothing and the caller uses ordinary memory.  Safe from any thread; a process forked by the
+// not; beyond that take() gives nothing and the caller uses ordinary memory.  Locking and unlocking takes milliseconds, so free
+// blocks make room for another size only when they are enough and that size is asked for twice in a row: 8 rows of 151,936 in
+// turn with 120, which fit no block, took 5 to 30 ms instead of 0.5 when every miss freed them.  Safe from any thread; a process forked by the
 // caller keeps its own copy of a result and leaves the pool alone.
 class QE_API RowPool {
 public:
@@ -102,10 +104,11 @@ public:
     static constexpr size_t kMost = (size_t)64 << 20;
     static Block* take(const std::shared_ptr<RowPool>& pool, size_t bytes);      // null: none to be had
     static void give(Block* block);
+    size_t held();
 private:
     std::mutex mutex_;
     std::vector<std::unique_ptr<Block>> free_;
-    size_t held_ = 0;
+    size_t held_ = 0, missed_ = 0;           // missed_: what the last take() found no room for (0: it found some)
 };
 
 class QE_API Engine {

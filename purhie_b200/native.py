@@ -210,6 +210,7 @@ _SIGNATURES = {
     "qe_profile_report": (c_char_p, [c_int]),
     "qe_rows_take": (c_void_p, [_P, c_longlong, POINTER(c_void_p)]),
     "qe_rows_give": (None, [c_void_p]),
+    "qe_rows_held": (c_longlong, [_P]),
     "qe_launches": (c_longlong, []),
     "qe_set_library_dir": (None, [c_char_p]),
 }

@@ -121,3 +121,40 @@ def test_a_forked_process_keeps_the_results_it_was_given():
     fresh.step([StepEntry("a", toks[:8], [])])
     assert np.array_equal(fresh.step([StepEntry("a", toks[8:16], range(8))]), again)
     fresh.close()
+
+
+def test_blocks_of_results_make_room_only_where_that_helps():
+    """Free blocks stay when a result fits nowhere (too large, or beside those in use), and when sizes that do not fit side by
+    side come in turn; a size that is asked for again gets their room."""
+    import ctypes
+    from purhie_b200 import native
+    from purhie_b200.engine import Engine
+    eng = Engine.from_random(TINY_C, 3, dtype="bfloat16", page_size=16, max_tokens=256, max_requests=1)
+    lib, MiB = native.lib(), 1 << 20
+    held = lambda: lib.qe_rows_held(eng._handle) // MiB
+
+    def take(size):
+        data = ctypes.c_void_p()
+        return lib.qe_rows_take(eng._handle, size * MiB, ctypes.byref(data)), data.value
+
+    a, where = take(8)
+    lib.qe_rows_give(a)
+    assert take(65) == (None, None) and take(65)[0] is None and held() == 8
+    a, again = take(8)
+    assert again == where
+    b, _ = take(40)
+    assert b and held() == 48
+    assert take(52)[0] is None and take(52)[0] is None and held() == 48       # (both blocks are in use)
+    lib.qe_rows_give(a)
+    assert take(52)[0] is None and take(52)[0] is None and held() == 48       # (eight are not enough)
+    lib.qe_rows_give(b)
+    for _ in range(3):                                                        # 52 and 40 in turn: 40 keeps its block
+        assert take(52)[0] is None
+        b, _ = take(40)
+        assert b and held() == 48
+        lib.qe_rows_give(b)
+    assert take(52)[0] is None
+    c, _ = take(50)                                                           # about the same size again
+    assert c and held() == 50
+    lib.qe_rows_give(c)
+    eng.close()
