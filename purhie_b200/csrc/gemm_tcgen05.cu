@@ -58,8 +58,8 @@ struct GemmParams {
     long long split_stride;
     // A factor per token that the norm in front left out of the activations, rsqrt(sum over the chunks of
     // row_sumsq[token][chunk] / row_width + row_eps), applied to the accumulator before anything else happens to it
-    // (the product is linear in its rows).  Swapped orientation: bfloat16 output; plain orientation: tiles of 256
-    // columns, one split, no accumulate.  Null: none.
+    // (the product is linear in its rows).  Swapped orientation: bfloat16 output; plain orientation: tiles of 64
+    // columns or more, one split, no accumulate.  Null: none.
     const float* row_sumsq;
     int row_chunks, row_width;
     float row_eps;
@@ -80,8 +80,8 @@ struct GemmParams {
     // null) multiplies the rows of the accumulator in front of the activation.
     const int32_t* tile_group;
     const float* row_factor;
-    // One-CTA kernel: the weight was complete before the kernel in front of this one started, so its first tiles are asked for
-    // before that kernel has ended.
+    // One-CTA kernel, plain orientation (tiles of 64 columns or more): the weight was complete before the kernel in front of this one started, so its first tiles
+    // are asked for before that kernel has ended (swapped: always).
     int early_w;
     int* error_flag;
 };
@@ -193,8 +193,9 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Few tokens (BN <= 64: weight streaming): two CTAs share an SM, each with half the stages, so that one CTA's
-// start-up and epilogue overlap the other's streaming.  Many tokens: one CTA per SM with all the stages.
+// Tiles of at most 64 on the B side (few tokens, whose product is weight streaming, and narrow tiles of many): two CTAs share an
+// SM, each with half the stages, so that one CTA's start-up and epilogue overlap the other's streaming.  Wider tiles: one CTA
+// per SM with all the stages.
 template <int BN> struct TileConfig {
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -474,9 +475,11 @@ __device__ __forceinline__ void store_chunk_swapped_bf16(const GemmParams& p, ui
     __syncwarp();                                      // the buffer is written again for the next chunk
 }
 
-// ROW_SCALE: the instance whose plain epilogue knows a factor per row (a register or two that the few-token instances of 64 and
-// 128 columns do without).
-template <int BN, bool ROW_SCALE>
+// What an instance is compiled with.  FEW: nothing that only many tokens need (with the two below in its code, a decode product of
+// 4.44 us took 4.48 to 4.52).  PLAIN: the plain walk can ask for its weight early.  SCALED: also, the plain epilogue knows a
+// factor per row.
+enum Instance { FEW, PLAIN, SCALED };
+template <int BN, Instance KIND>
 __global__ void __launch_bounds__(NUM_THREADS, TileConfig<BN>::CTAS_PER_SM)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmParams p) {
     using Cfg = TileConfig<BN>;
@@ -537,16 +540,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             wb.start(blockIdx.x, work_total);
             int pre = 0;
             // fill the (still empty) ring with tiles of the weight now: A in the swapped orientation, B in the plain one
-            for (; p.early_w && pre < STAGES && wa.valid; ++pre) {
-                mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
-                if (p.swapped) tma_load_2d(smem_a + pre * A_BYTES, &map_a, &full[pre], wa.kb * BK, wa.a0);
-                else tma_load_2d(smem_b + pre * Cfg::B_BYTES, &map_b, &full[pre], wa.kb * BK, wa.b0);
-                wa.next(gridDim.x, work_total);
+            const bool early_b = KIND != FEW && !p.swapped;
+            if (p.swapped) {
+                for (; pre < STAGES && wa.valid; ++pre) {
+                    mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
+                    tma_load_2d(smem_a + pre * A_BYTES, &map_a, &full[pre], wa.kb * BK, wa.a0);
+                    wa.next(gridDim.x, work_total);
+                }
+            } else if (early_b && p.early_w) {
+                for (; pre < STAGES && wa.valid; ++pre) {
+                    mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
+                    tma_load_2d(smem_b + pre * Cfg::B_BYTES, &map_b, &full[pre], wa.kb * BK, wa.b0);
+                    wa.next(gridDim.x, work_total);
+                }
             }
             pdl_wait();
             for (int s = 0; s < pre; ++s) {                  // the activation tiles of those stages
-                if (p.swapped) tma_load_2d(smem_b + s * Cfg::B_BYTES, &map_b, &full[s], wb.kb * BK, wb.b0);
-                else tma_load_2d(smem_a + s * A_BYTES, &map_a, &full[s], wb.kb * BK, wb.a0);
+                if (early_b) tma_load_2d(smem_a + s * A_BYTES, &map_a, &full[s], wb.kb * BK, wb.a0);
+                else tma_load_2d(smem_b + s * Cfg::B_BYTES, &map_b, &full[s], wb.kb * BK, wb.b0);
                 wb.next(gridDim.x, work_total);
             }
             int stage = pre == STAGES ? 0 : pre;
@@ -625,10 +636,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             // the norm ahead (tiles of 256 columns)
             const int a = a0 + q * 32 + lane;
             constexpr bool ROW_OPS = BN == 256;
-            const bool scale_row = ROW_SCALE && !p.swapped && p.row_sumsq != nullptr;
+            const bool scale_row = KIND == SCALED && !p.swapped && p.row_sumsq != nullptr;
             float row_f = 1.0f;
             float ss[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if constexpr (ROW_SCALE) row_f = scale_row ? plain_row_factor(p, a) : 1.0f;
+            if constexpr (KIND == SCALED) row_f = scale_row ? plain_row_factor(p, a) : 1.0f;
             if (!mbar_wait(&acc_full[acc], acc_phase, p.error_flag, PH_ERR_WAIT_EPILOGUE)) { ok = false; break; }
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
@@ -649,7 +660,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
                 if constexpr (CH == 32) tmem_ld32(taddr + c, r); else tmem_ld16(taddr + c, r);
                 tmem_ld_wait();
-                if constexpr (ROW_SCALE) {
+                if constexpr (KIND == SCALED) {
                     if (scale_row) {
 #pragma unroll
                         for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * row_f);
@@ -1105,11 +1116,11 @@ int sm_count() {
     return n;
 }
 
-template <int BN, bool ROW_SCALE>
+template <int BN, Instance KIND>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int max_ctas, cudaStream_t stream) {
     using Cfg = TileConfig<BN>;
     static bool configured = false;
-    auto kernel = gemm_tcgen05_kernel<BN, ROW_SCALE>;
+    auto kernel = gemm_tcgen05_kernel<BN, KIND>;
     if (!configured) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
             return fail(PH_ERR_LAUNCH, "gemm_tcgen05: cannot reserve %d bytes of shared memory", Cfg::SMEM_BYTES);
@@ -1257,7 +1268,7 @@ PH_EXPORT int ph_gemm_bf16_tcgen05_grouped(const void* x, const void* w, void* o
 // (the formula of src/gpu_ops.hip:103-114 in the reference).
 // accumulate: out (float32, plain orientation, one split, no activation) += the product.
 // row_sumsq [M][row_chunks] (or null), row_width, row_eps: the activations lack a factor per token, see GemmParams;
-// taken by the swapped orientation with bfloat16 output, and by the plain orientation with tiles of 256 columns.
+// taken by the swapped orientation with bfloat16 output, and by the plain orientation with tiles of 64 columns or more.
 // norm_weight, norm_rows, norm_sumsq: as in the pair kernel (plain orientation, block_n 256, accumulate).
 // early_w: w is not a result of the kernel in front on the stream, nor of one that may still run then, and its first tiles may
 // be read before that kernel has ended.  The swapped orientation always does that: its w has to be such a weight.
@@ -1305,14 +1316,15 @@ PH_EXPORT int ph_gemm_bf16_tcgen05(const void* x, const void* w, void* out, int 
     p.row_sumsq = row_sumsq; p.row_chunks = row_chunks; p.row_width = row_width; p.row_eps = row_eps;
     p.norm_weight = norm_weight; p.norm_rows = (__nv_bfloat16*)norm_rows; p.norm_sumsq = norm_sumsq;
     p.tma_store = 0;
-    p.early_w = swapped || early_w;
-    const bool scaled = !swapped && row_sumsq != nullptr;
+    p.early_w = early_w;
     switch (block_n) {
-        case 16: return launch<16, false>(ma, mb, p, max_ctas, stream);
-        case 32: return launch<32, false>(ma, mb, p, max_ctas, stream);
-        case 64: return scaled ? launch<64, true>(ma, mb, p, max_ctas, stream) : launch<64, false>(ma, mb, p, max_ctas, stream);
-        case 128: return scaled ? launch<128, true>(ma, mb, p, max_ctas, stream) : launch<128, false>(ma, mb, p, max_ctas, stream);
-        case 256: return launch<256, true>(ma, mb, p, max_ctas, stream);
+        case 16: return launch<16, FEW>(ma, mb, p, max_ctas, stream);
+        case 32: return launch<32, FEW>(ma, mb, p, max_ctas, stream);
+        case 64: return swapped ? launch<64, FEW>(ma, mb, p, max_ctas, stream)
+                                : row_sumsq ? launch<64, SCALED>(ma, mb, p, max_ctas, stream) : launch<64, PLAIN>(ma, mb, p, max_ctas, stream);
+        case 128: return swapped ? launch<128, FEW>(ma, mb, p, max_ctas, stream)
+                                 : row_sumsq ? launch<128, SCALED>(ma, mb, p, max_ctas, stream) : launch<128, PLAIN>(ma, mb, p, max_ctas, stream);
+        case 256: return launch<256, SCALED>(ma, mb, p, max_ctas, stream);
         default: return fail(PH_ERR_ARG, "gemm_tcgen05: block_n %d is not one of 16, 32, 64, 128, 256", block_n);
     }
 }
