@@ -19,6 +19,7 @@
 // (rows of HQ * DV logits, or none) multiplies the output by sigmoid(gate), element by element.
 // Formulas (reference): src/qwen_ops.cpp:26-51 (scores * scale, max-subtracted softmax, weighted sum of
 // V; query head h uses kv head h / (HQ / HKV)); window: src/attention.h:73.
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "shared_limit.cuh"
 
@@ -131,13 +132,6 @@ struct F32Params {
 constexpr int RUN_MIN = 4;           // tokens of one request side by side that the tile kernel takes
 constexpr int FEW_ROWS_PER_SM = 64;  // (token, head) rows an SM below which a warp of the tile kernel takes four instead of eight
 constexpr int KEYS = 128;            // keys a CTA of the rows kernel scores at once
-
-__device__ __forceinline__ void copy16(float* dst, const float* src) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // The score of a key from its dot product, every operation rounded by itself as in the plain kernel.
 __device__ __forceinline__ float bent_score(float dot, float scale, float cap, bool biased, float slope, int distance) {

@@ -15,6 +15,7 @@
 // a tiny model's three streams of 12 tokens 1.78 -> 1.64 ms).  Elsewhere, started early, their CTAs pile up on the SMs that the kernel in
 // front leaves first, and with one or two CTAs an SM that imbalance cost a 256-row layer of a 0.6B
 // model 61 us (428 against 367).
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "shared_limit.cuh"
 
@@ -83,14 +84,8 @@ __global__ void __launch_bounds__(256) gemm_simple_kernel(const TX* __restrict__
 
 // ---- float32: 16-byte asynchronous copies --------------------------------------------------------------------------
 // A row of an operand in shared memory holds its k side by side, padded by 16 bytes: eight neighbouring rows then start
-// in eight different groups of four banks, so a warp whose lanes read float4s of eight rows (the same k) has no conflict.
-__device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    const int n = valid ? 16 : 0;                                  // nothing valid: zeros are written, src is not read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// in eight different groups of four banks, so lanes that read float4s of eight rows (the same k) ask for every bank once.
+// (The counters show about three wavefronts for such a read in gemm_tile_f32 all the same.)
 
 // Few rows.  A CTA owns BN_ columns and all MB rows: its 128 threads keep STAGES chunks of KC numbers of its weight rows (and
 // of x) on their way, and BN_ * MB / RM of them multiply, one column and RM rows each.  What bounds it: the chain of K
@@ -173,7 +168,7 @@ __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(const float* __restr
 }
 
 // Many rows.  A CTA of two warps owns 32 x 32 outputs, a thread 4 x 4 of them, its rows and columns interleaved with its
-// neighbours' (lanes: 8 columns x 4 rows), so that four k of eight rows are one conflict-free access.  Both operands keep k
+// neighbours' (lanes: 8 columns x 4 rows), so that a read takes four k of eight rows and no bank twice.  Both operands keep k
 // contiguous in shared memory, which cp.async can write without a transposition through registers.  What bounds it: the
 // shared-memory reads (81 % of their rate at 1024 x 6144 x 1024) and the issue of the multiply-adds (68 %).  Many small CTAs
 // that wait for their own copies only are as fast as larger tiles where there are many outputs (1024 x 6144 x 1024: 319 us,

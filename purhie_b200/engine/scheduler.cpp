@@ -83,8 +83,8 @@ int Scheduler::largest_portion(const GenRequest& r, int want, const std::vector<
 
 // The portion of n tokens (of `rest` that the request still has) after `used` rows of the step: when the prompt
 // goes on after it and the step would end past a multiple of align_rows, the portion ends there instead, unless
-// that takes more than half of it.  (The products run in tiles of that many rows: a step of 544 rows costs what
-// one of 768 does.)
+// that takes more than half of it.  (Most products run in tiles of that many rows, and a step of 544 rows costs
+// about what one of 768 does: the products of an 8B layer 233 and 256 us, of a 0.6B layer 49 and 48; 512 rows 181 and 43.)
 int Scheduler::aligned(int n, int rest, int used) const {
     const int a = align_rows_;
     if (!a || n >= rest || used + n < a) return n;
