@@ -10,7 +10,7 @@
 //   route_sort     the (token, choice) pairs sorted by expert: position of each pair, pair at each position, and a
 //                  list of row tiles (expert, first position, rows) that never cross from one expert to the next.
 //   gemm_grouped   y[i] = W[expert of i] x[source row of i] for the sorted positions i, tile by tile; float32
-//                  multiply-add on the CUDA cores with k ascending inside one thread (the order of gemm_simple),
+//                  multiply-add on the CUDA cores with k ascending inside one thread,
 //                  so a row's result depends on neither its place in the batch nor its place among the expert's rows.
 //   gemv_grouped   the same product for a handful of rows per expert (decoding): a warp per output feature streams
 //                  that feature's weight row once, 16 bytes per lane and load, for up to eight rows of the tile at a

@@ -36,6 +36,14 @@ def test_float32_product_adds_in_the_plain_kernels_order(M, N, K):
     assert ((out.double() - x.double() @ w.double().T).abs() <= bound).all()
 
 
+# K shared out among warps (three blocks of 128 and more): a round that is full, one that is not, a block of four numbers; columns up
+# to the most that the few-row form takes; tiles in four groups, in two and in one
+@pytest.mark.parametrize("M", [1, 2, 4, 7, 8, 16, 32, 139, 300])
+@pytest.mark.parametrize("N,K", [(9, 260), (64, 1024), (1000, 3076), (2368, 388), (8200, 300)])
+def test_float32_product_shares_k_out_in_the_plain_kernels_order(M, N, K):
+    test_float32_product_adds_in_the_plain_kernels_order(M, N, K)
+
+
 # decoded tokens alone (rows kernel), portions long enough for tiles beside decoded tokens, a portion of three tokens, portions
 # that start mid-context; block edges of 32 and 128 keys; enough rows for tiles of eight rows a warp
 CASES = [[(1, 1), (32, 1), (33, 1), (128, 1), (129, 1), (300, 1)],
