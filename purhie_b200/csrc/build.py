@@ -48,6 +48,12 @@ LIBRARIES: Dict[str, dict] = {
         "flags": [],
         "link": [],
     },
+    "layers": {
+        "sources": ["decode_layers.cu"],
+        "deps": ["attention_mma.cuh", "decode_layers.h", "mbarrier.cuh"],
+        "flags": [],
+        "link": [],
+    },
     "gemm100": {
         "sources": ["gemm_tcgen05.cu"],
         "flags": [],
@@ -60,13 +66,13 @@ LIBRARIES: Dict[str, dict] = {
                     "../parts/registry.cpp", "../parts/linear.cpp", "../parts/norm.cpp", "../parts/rotary.cpp",
                     "../parts/attention.cpp", "../parts/feed_forward.cpp", "../parts/routed.cpp", "../parts/mamba.cpp",
                     "../parts/linear_attention.cpp", "../parts/latent_attention.cpp", "../parts/embedding.cpp", "../parts/block.cpp",
-                    "../parts/min_gru.cpp", "../parts/delta_rule.cpp", "../config/bozosun.cpp", "../config/sizizen.cpp", "../config/zerusun.cpp", "../config/vokepel.cpp",
+                    "../parts/min_gru.cpp", "../parts/delta_rule.cpp", "../parts/decode_stack.cpp", "../config/bozosun.cpp", "../config/sizizen.cpp", "../config/zerusun.cpp", "../config/vokepel.cpp",
                     "../config/noditar.cpp", "../config/defapel.cpp",
                     "../parts/model.cpp", "../cache/cache.cpp", "../sampling/sampler.cpp", "../engine/engine.cpp",
                     "../engine/scheduler.cpp", "../api/capi.cpp", "../api/capi_generate.cpp", "../api/test_hooks.cpp",
                     "../api/test_hooks_host.cpp", "../api/test_hooks_parts.cpp"],
         "deps": ["../host/common.h", "../host/json.h", "../host/device.h", "../config/config.h", "../weights/safetensors.h",
-                 "../weights/weights.h", "../weights/random.h", "../parts/parts.h", "../parts/linear.h", "../parts/gate.h", "../parts/model.h",
+                 "../weights/weights.h", "../weights/random.h", "../parts/parts.h", "../parts/linear.h", "../parts/gate.h", "../parts/model.h", "../parts/decode_stack.h", "decode_layers.h",
                  "../cache/cache.h", "../sampling/sampler.h", "../engine/engine.h", "../engine/scheduler.h",
                  "../api/inference.h", "../api/capi_internal.h"],
         "flags": ["-Xcompiler", "-ffp-contract=off"],

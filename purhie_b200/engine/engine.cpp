@@ -32,7 +32,10 @@ std::string flag_text(int which, int code) {
                   : code == 112 ? "an attention consumer waited too long for keys"
                   : code == 121 ? "the prefill attention producer waited too long"
                   : code == 122 ? "the prefill attention tensor-core warp waited too long"
-                  : code == 123 ? "a prefill attention softmax warp waited too long" : "error";
+                  : code == 123 ? "a prefill attention softmax warp waited too long"
+                  : code == 131 ? "a copying warp of the one-launch decode step waited too long for a free place"
+                  : code == 132 ? "a warp of the one-launch decode step waited too long for its operands"
+                  : code == 133 ? "a CTA of the one-launch decode step waited too long for the others" : "error";
     return "attention kernel: " + std::string(t) + " (status " + std::to_string(code) + ")";
 }
 }  // namespace
@@ -50,6 +53,7 @@ Engine::Engine(std::shared_ptr<DecoderModel> model, const EngineOptions& options
     cache_.reset(new CacheManager(model_->cache_needs(), options_.page_size, pages, options_.max_requests));
     cache_->materialize(model_->compute_dtype(), options_.poison_cache, stream_);
     views_ = model_->cache_views(*cache_);
+    decode_stack_ = DecodeStack::make(model_->decode_layers(), views_, stream_);
     row_multiple_ = model_->compute_dtype() == DType::BF16 ? model_->preferred_row_multiple() : 0;
     for (int i = 0; i < 2; i++) QE_CUDA(cudaEventCreateWithFlags(&meta_event_[i], cudaEventDisableTiming));
     error_words_ = DeviceBuffer(16);
@@ -206,6 +210,7 @@ void Engine::context(const Layout& lay, const int32_t* dev, Workspace& ws, StepC
     ctx.gemm_error = static_cast<int*>(error_words_.data());
     ctx.attention_error = static_cast<int*>(error_words_.data()) + 1;
     ctx.options = &options_.step_options;
+    ctx.decode_stack = decode_stack_.get();
 }
 
 void context_from_layout(const StepLayout& lay, const CacheManager& cache, int position_columns, const int32_t* dev, StepContext& ctx,

@@ -25,6 +25,7 @@
 
 #include "../cache/cache.h"
 #include "../config/config.h"
+#include "../parts/decode_stack.h"
 #include "../parts/model.h"
 #include "../sampling/sampler.h"
 #include "../weights/weights.h"
@@ -200,6 +201,7 @@ private:
     std::shared_ptr<RowPool> row_pool_ = std::make_shared<RowPool>();
     std::unique_ptr<CacheManager> cache_;
     std::vector<CacheView> views_;
+    std::unique_ptr<DecodeStack> decode_stack_;          // null: the model's layers do not fit it
     Workspace workspace_;
     cudaStream_t stream_ = nullptr;
     int row_multiple_ = 0;

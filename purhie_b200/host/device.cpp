@@ -108,7 +108,8 @@ CoreKernels g_core{};
 FlashKernels g_flash{};
 GemmKernels g_gemm{};
 LatentKernels g_latent{};
-bool g_core_ok = false, g_flash_ok = false, g_gemm_ok = false, g_latent_ok = false;
+LayersKernels g_layers{};
+bool g_core_ok = false, g_flash_ok = false, g_gemm_ok = false, g_latent_ok = false, g_layers_ok = false;
 
 std::string own_dir() {
     Dl_info info;
@@ -275,11 +276,28 @@ const LatentKernels& latent_kernels() {
     return g_latent;
 }
 
+const LayersKernels& layers_kernels() {
+    if (g_layers_ok) return g_layers;
+    std::lock_guard<std::mutex> lock(g_lib_mutex);
+    if (g_layers_ok) return g_layers;
+    void* h = open_library("layers");
+    bind(h, "layers", "ph_decode_layers_supports", g_layers.supports);
+    bind(h, "layers", "ph_decode_layers_shares", g_layers.shares);
+    bind(h, "layers", "ph_decode_layers_counters", g_layers.counters);
+    bind(h, "layers", "ph_decode_layers_map", g_layers.map);
+    bind(h, "layers", "ph_decode_layers_weight_map", g_layers.weight_map);
+    bind(h, "layers", "ph_decode_layers", g_layers.decode_layers);
+    bind(h, "layers", "ph_layers_last_error", g_layers.last_error);
+    g_layers_ok = true;
+    return g_layers;
+}
+
 void require_library(const std::string& name) {
     if (name == "core") core_kernels();
     else if (name == "flash") flash_kernels();
     else if (name == "gemm100") gemm_kernels();
     else if (name == "latent") latent_kernels();
+    else if (name == "layers") layers_kernels();
     else {
         std::lock_guard<std::mutex> lock(g_lib_mutex);
         open_library(name);

@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "../csrc/decode_layers.h"
 #include "common.h"
 
 namespace qe {
@@ -295,6 +296,15 @@ struct GemmKernels {
                         cudaStream_t);
     const char* (*last_error)(void);
 };
+struct LayersKernels {
+    int (*supports)(int, int, int, int, int, int, int, int, int);
+    int (*shares)(int, int, int, int, int, int32_t*);
+    int (*counters)(int, int);
+    int (*map)(void*, const void*, const void*, long long, int, int, int, int*);
+    int (*weight_map)(void*, const void*, int, int);
+    int (*decode_layers)(const PhDecodeLayersArgs*, cudaStream_t);
+    const char* (*last_error)(void);
+};
 
 // Folder the kernel libraries are opened from: set_library_dir(), else $PURHIE_B200_LIB_DIR, else the folder
 // this library itself was loaded from.
@@ -304,7 +314,8 @@ QE_API const CoreKernels& core_kernels();
 QE_API const FlashKernels& flash_kernels();
 QE_API const GemmKernels& gemm_kernels();
 QE_API const LatentKernels& latent_kernels();
-QE_API void require_library(const std::string& name);      // "core", "flash", "gemm100", "latent": open it now
+QE_API const LayersKernels& layers_kernels();
+QE_API void require_library(const std::string& name);      // "core", "flash", "gemm100", "latent", "layers": open it now
 QE_API extern long long g_launches;                          // launcher calls so far (for the bench's count)
 
 // Time per kernel class, for finding out where a step's time goes (the reference prints such a breakdown under

@@ -335,6 +335,18 @@ public:
         return compute_dtype == DType::BF16 && takes(qkv_proj_) && (!q_only_proj_.defined() || takes(q_only_proj_));
     }
 
+    bool decode_layer(DecodeLayerSpec& d) const override {
+        if (!use_flash() || extended() || !has_norm_ || row_norm_ || has_bias_ || value_mix_ || reach() || !position_ || position_->interleaved() ||
+            position_->n_rot() != head_dim_ || !table_.defined() || value_dim_ != head_dim_ || !qkv_proj_.fast() || !o_proj_.fast())
+            return false;
+        d.w_qkv = qkv_proj_.weight().data; d.w_o = o_proj_.weight().data;
+        d.q_norm = q_norm_.as<float>(); d.k_norm = k_norm_.as<float>();
+        d.rotation = table_.as<float>(); d.max_position = table_.shape[0]; d.position_column = position_->position_column();
+        d.width = hidden_; d.heads = heads_; d.kv_heads = kv_heads_; d.head_dim = head_dim_;
+        d.qk_eps = (float)eps_; d.scale = (float)scale_;
+        return true;
+    }
+
     // ---- step ----------------------------------------------------------------------------------------------------
     Addend forward(const Tensor& x, StepContext& ctx, const CacheView& cache) override {
         const int T = ctx.T;

@@ -80,6 +80,11 @@ public:
         const bool may_defer = ctx.option("row_factor") != "norm";
         return factor_ == 1.0f && may_defer && mixer_->takes_unscaled_rows(ctx) ? mixer_norm_->offer(ctx) : NormAhead();
     }
+    bool decode_layer(DecodeLayerSpec& d) const override {
+        float second = 0.0f;
+        return factor_ == 1.0f && ff_ && mixer_norm_->plain_rms(&d.norm1, &d.norm_eps) && ff_norm_->plain_rms(&d.norm2, &second) &&
+               second == d.norm_eps && mixer_->decode_layer(d) && ff_->decode_layer(d);
+    }
 private:
     // What a part gives is multiplied by the factor on its way into the residual, so no product adds into the residual
     // itself and no norm's work is handed to a product: every part returns its addend, which carries the factor.

@@ -1,0 +1,112 @@
+#include "decode_stack.h"
+
+#include "../csrc/decode_layers.h"
+
+namespace qe {
+
+namespace {
+constexpr int kMostRows = 8;
+DeviceBuffer upload(const void* host, size_t bytes, cudaStream_t stream) {
+    DeviceBuffer b(bytes);
+    QE_CUDA(cudaMemcpyAsync(b.data(), host, bytes, cudaMemcpyHostToDevice, stream));
+    QE_CUDA(cudaStreamSynchronize(stream));
+    return b;
+}
+}  // namespace
+
+std::unique_ptr<DecodeStack> DecodeStack::make(const std::vector<DecodeLayerSpec>& layers, const std::vector<CacheView>& views, cudaStream_t stream) {
+    if (layers.empty() || layers.size() != views.size()) return nullptr;
+    const DecodeLayerSpec& a = layers[0];
+    const CacheView& v = views[0];
+    for (size_t i = 0; i < layers.size(); i++) {
+        const DecodeLayerSpec& b = layers[i];
+        const CacheView& w = views[i];
+        if (b.width != a.width || b.inner != a.inner || b.heads != a.heads || b.kv_heads != a.kv_heads || b.head_dim != a.head_dim ||
+            b.norm_eps != a.norm_eps || b.qk_eps != a.qk_eps || b.scale != a.scale || b.rotation != a.rotation ||
+            b.max_position != a.max_position || b.position_column != a.position_column)
+            return nullptr;
+        if (w.kind != CacheNeed::Pages || !w.writable || w.kv_dtype != DType::BF16 || w.group != v.group || w.page_size != v.page_size ||
+            w.page_stride != v.page_stride || w.num_pages != v.num_pages || w.num_pages < 1 || w.kv_heads != a.kv_heads || w.key_dim != a.head_dim ||
+            w.value_dim != a.head_dim || w.state.defined())
+            return nullptr;
+    }
+    const LayersKernels& k = layers_kernels();
+    std::unique_ptr<DecodeStack> s(new DecodeStack());
+    s->first_ = a;
+    s->n_layers_ = (int)layers.size();
+    s->group_ = v.group; s->page_size_ = v.page_size; s->page_stride_ = v.page_stride;
+    s->num_ctas_ = sm_count();
+    std::vector<int32_t> shares((size_t)4 * (s->num_ctas_ + 1));
+    s->most_groups_ = k.shares((int)a.width, a.heads, a.kv_heads, (int)a.inner, s->num_ctas_, shares.data());
+    if (!k.supports(1, (int)a.width, a.heads, a.kv_heads, a.head_dim, (int)a.inner, v.page_size, s->n_layers_, s->most_groups_)) return nullptr;
+    std::vector<PhDecodeLayer> records;
+    constexpr int kMaps = 5;                              // of a layer: four weights, the cache entry; 128 bytes each
+    std::vector<uint8_t> maps((size_t)kMaps * 128 * layers.size());
+    const int qkv = (a.heads + 2 * a.kv_heads) * a.head_dim, q = a.heads * a.head_dim, E = (int)a.width, F = (int)a.inner;
+    for (size_t i = 0; i < layers.size(); i++) {
+        const DecodeLayerSpec& b = layers[i];
+        records.push_back({b.norm1, b.norm2, b.q_norm, b.k_norm, views[i].k_base, views[i].v_base});
+        uint8_t* m = maps.data() + (size_t)kMaps * 128 * i;
+        if (k.weight_map(m, b.w_qkv, qkv, E) != 0 || k.weight_map(m + 128, b.w_o, E, q) != 0 || k.weight_map(m + 256, b.w_gate_up, 2 * F, E) != 0 ||
+            k.weight_map(m + 384, b.w_down, E, F) != 0 ||
+            k.map(m + 512, views[i].k_base, views[i].v_base, v.page_stride, v.page_size, v.num_pages, a.kv_heads, &s->total_rows_) != 0)
+            return nullptr;
+    }
+    s->layers_ = upload(records.data(), records.size() * sizeof(PhDecodeLayer), stream);
+    s->maps_ = upload(maps.data(), maps.size(), stream);
+    s->shares_ = upload(shares.data(), shares.size() * 4, stream);
+    const std::vector<int32_t> zeros((size_t)k.counters(s->n_layers_, a.kv_heads), 0);
+    s->counters_ = upload(zeros.data(), zeros.size() * 4, stream);
+    return s;
+}
+
+bool DecodeStack::takes(const StepContext& ctx) const {
+    if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T) return false;
+    if (ctx.options && ctx.options->is_object() && !ctx.options->members().empty()) return false;
+    return layers_kernels().supports(ctx.T, (int)first_.width, first_.heads, first_.kv_heads, first_.head_dim, (int)first_.inner, page_size_, n_layers_,
+                                     most_groups_) != 0;
+}
+
+void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
+    const int T = ctx.T, group = first_.heads / first_.kv_heads;
+    const int64_t E = first_.width, D = first_.head_dim, pieces = num_ctas_;
+    Workspace& ws = *ctx.workspace;
+    const GroupStep& g = ctx.groups.at(group_);
+    PhDecodeLayersArgs a{};
+    a.layers = static_cast<const PhDecodeLayer*>(layers_.data());
+    a.maps = maps_.data();
+    a.shares = static_cast<const int32_t*>(shares_.data());
+    a.counters = static_cast<int32_t*>(counters_.data());
+    a.n_layers = n_layers_; a.width = (int)E; a.heads = first_.heads; a.kv_heads = first_.kv_heads; a.inner = (int)first_.inner;
+    a.page_size = page_size_; a.total_rows = total_rows_; a.max_position = (int)first_.max_position;
+    a.most_groups = most_groups_; a.page_stride = page_stride_;
+    a.norm_eps = first_.norm_eps; a.qk_eps = first_.qk_eps; a.scale = first_.scale;
+    a.rotation = first_.rotation;
+    a.rows = T;
+    a.block_table = g.block_table; a.table_width = g.table_width;
+    a.row_seg = ctx.row_seg;
+    a.positions = ctx.position_column(0);
+    a.rotation_positions = ctx.position_column(first_.position_column);
+    a.slots = g.slot_mapping;
+    a.x = stream.x.as<float>();
+    a.xw = ws.get("stack_xw", {T, E}, DType::BF16).data;
+    a.sumsq = ws.get("stack_sumsq", {T, E / 16}, DType::F32).as<float>();
+    a.qkv = ws.get("stack_qkv", {T, (first_.heads + 2 * first_.kv_heads) * D}, DType::F32).as<float>();
+    a.attn = ws.get("stack_attn", {T, first_.heads * D}, DType::BF16).data;
+    a.act = ws.get("stack_act", {T, first_.inner}, DType::BF16).data;
+    a.part_o = ws.get("stack_part_o", {pieces, group, D}, DType::F32).as<float>();
+    a.part_ml = ws.get("stack_part_ml", {pieces, group, 2}, DType::F32).as<float>();
+    a.error_flag = ctx.attention_error;
+    if (LaunchProfile::get().on()) {
+        const double weights = (double)E * (first_.heads + 2 * first_.kv_heads) * D + (double)first_.heads * D * E + 3.0 * E * first_.inner;
+        double keys = 0.0;
+        for (int len : ctx.ctx_lens) keys += len;
+        LaunchProfile::get().note_cost(n_layers_ * (2.0 * weights + keys * 4.0 * first_.kv_heads * D),
+                                       n_layers_ * (2.0 * T * weights + keys * 4.0 * first_.heads * D));
+    }
+    const LayersKernels& k = layers_kernels();
+    QE_LAUNCH(k, k.decode_layers(&a, ctx.stream));
+    stream.clear();
+}
+
+}  // namespace qe

@@ -1,0 +1,32 @@
+// All layers of a decode step of a few rows as one launch (csrc/decode_layers.cu): what is fixed for a model and its cache, and
+// which steps take it.
+//
+// Models whose every layer is pre-norm with RMS norms, attention with a norm per head of 128 and half-pair rotation over all
+// earlier positions, and a SwiGLU feed-forward, all in bfloat16.  Steps of at most eight requests with one token each.
+#pragma once
+
+#include <memory>
+#include <vector>
+
+#include "parts.h"
+
+namespace qe {
+
+class QE_API DecodeStack {
+public:
+    // Null when the layers or the cache entries do not fit.
+    static std::unique_ptr<DecodeStack> make(const std::vector<DecodeLayerSpec>& layers, const std::vector<CacheView>& views, cudaStream_t stream);
+    // Whether this step goes through the one launch.  The option "decode_stack": "off" keeps a launch per operation, and a step
+    // with any other kernel choice among its options is made of the kernels it chooses.
+    bool takes(const StepContext& ctx) const;
+    // Every layer over the rows of stream.x, in place; nothing is pending afterwards.
+    void run(ResidualStream& stream, StepContext& ctx) const;
+private:
+    DecodeStack() = default;
+    DecodeLayerSpec first_;
+    int n_layers_ = 0, group_ = 0, page_size_ = 0, total_rows_ = 0, most_groups_ = 0, num_ctas_ = 0;
+    long long page_stride_ = 0;
+    DeviceBuffer layers_, maps_, shares_, counters_;
+};
+
+}  // namespace qe

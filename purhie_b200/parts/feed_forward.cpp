@@ -52,6 +52,13 @@ public:
         return compute_dtype == DType::BF16 && gate_up_.applies_row_scale(ctx.T, compute_dtype, true);
     }
 
+    bool decode_layer(DecodeLayerSpec& d) const override {
+        if (compute_dtype != DType::BF16 || gate_.kind || hidden_ != d.width || !gate_up_.fast() || !down_.fast()) return false;
+        d.w_gate_up = gate_up_.weight().data; d.w_down = down_.weight().data;
+        d.inner = inter_;
+        return true;
+    }
+
     Addend forward(const Tensor& x, StepContext& ctx) override {
         const int T = ctx.T;
         // where the tensor-core product runs, its epilogue applies the gate (either family); else a kernel behind it does

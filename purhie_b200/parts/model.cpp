@@ -1,5 +1,7 @@
 #include "model.h"
 
+#include "decode_stack.h"
+
 #include <algorithm>
 #include <set>
 
@@ -81,6 +83,17 @@ std::vector<CacheView> DecoderModel::cache_views(const CacheManager& manager) co
     return views;
 }
 
+std::vector<DecodeLayerSpec> DecoderModel::decode_layers() const {
+    std::vector<DecodeLayerSpec> out;
+    if (spec_.residual_lanes || build_.compute_dtype != DType::BF16) return out;
+    for (const LayerCall& call : spec_.schedule) {
+        DecodeLayerSpec d;
+        if (call.cache_from >= 0 || !layers_[call.layer]->decode_layer(d)) return {};
+        out.push_back(d);
+    }
+    return out;
+}
+
 int DecoderModel::preferred_row_multiple() const {
     int m = 0;
     for (Part* p : all_parts()) m = std::max(m, p->preferred_row_multiple());
@@ -103,7 +116,9 @@ Tensor DecoderModel::forward(StepContext& ctx, const std::vector<CacheView>& vie
         QE_CUDA(cudaMemcpyAsync(kept.data, stream.x.data, stream.x.bytes(), cudaMemcpyDeviceToDevice, ctx.stream));
         ctx.embedding_output = kept.as<float>();
     }
-    for (size_t i = 0; i < spec_.schedule.size(); i++) {
+    const bool one_launch = ctx.decode_stack && !after_entry && ctx.decode_stack->takes(ctx);
+    if (one_launch) ctx.decode_stack->run(stream, ctx);
+    for (size_t i = 0; i < spec_.schedule.size() && !one_launch; i++) {
         ctx.pass = spec_.schedule[i].pass;
         // a layer learns which norm the next entry of the run order starts with: its last product may work ahead for it
         ctx.next_layer_norm = i + 1 < spec_.schedule.size() ? layers_[spec_.schedule[i + 1].layer]->first_norm(ctx) : NormAhead();

@@ -31,6 +31,8 @@ public:
     // ---- cache
     std::vector<CacheNeed> cache_needs() const;              // one per entry of the run order (a borrower needs nothing itself)
     std::vector<CacheView> cache_views(const CacheManager& manager) const;
+    // The run order as the one-launch decode step sees it; empty if any entry does not fit.
+    std::vector<DecodeLayerSpec> decode_layers() const;
 
     // ---- step
     int preferred_row_multiple() const;

@@ -119,6 +119,12 @@ public:
         weight_ = shifted;
     }
 
+    bool plain_rms(const float** weight, float* eps) const override {
+        *weight = weight_.as<float>();
+        *eps = (float)eps_;
+        return true;
+    }
+
     Tensor forward(ResidualStream& stream, StepContext& ctx, const int32_t* rows, int n_rows) override {
         const int n = rows ? n_rows : ctx.T;
         // an addend whose transform is a factor alone is folded in by this norm's own kernel; a norm on the addend, or a

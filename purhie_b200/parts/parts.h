@@ -224,6 +224,18 @@ struct NormAhead {
     bool done() const { return rows.defined(); }
 };
 
+// A layer as the one-launch decode step sees it (decode_stack.h): a part that fits fills in its share, one that does not
+// says so.
+struct DecodeLayerSpec {
+    const void *w_qkv = nullptr, *w_o = nullptr, *w_gate_up = nullptr, *w_down = nullptr;
+    const float *norm1 = nullptr, *norm2 = nullptr, *q_norm = nullptr, *k_norm = nullptr, *rotation = nullptr;
+    int64_t width = 0, inner = 0, max_position = 0;
+    int heads = 0, kv_heads = 0, head_dim = 0, position_column = 0;
+    float norm_eps = 0.0f, qk_eps = 0.0f, scale = 0.0f;
+};
+
+class DecodeStack;
+
 struct StepContext {
     int T = 0, S = 0;
     const int32_t* token_ids = nullptr;      // [T]
@@ -253,6 +265,7 @@ struct StepContext {
     int pass = 0;                            // LayerCall::pass of the run-order entry that is running
     const float* embedding_output = nullptr; // [T, E] float32, what the embedding gave (only where the model keeps it)
     std::map<std::string, StepArray> arrays; // what parts added through StepPlan, by name
+    const DecodeStack* decode_stack = nullptr;   // the model's layers as one launch, where they and the cache allow that
     const Json* options = nullptr;           // kernel choices for tests ("decode_kernel": "cp_async", ...)
 
     const int32_t* position_column(int c) const { return positions + (size_t)c * T; }
@@ -381,6 +394,8 @@ public:
     // This norm as a transform of an addend (AddendTransform) with the given factor, for a layer that norms what a
     // part gives before adding it; a norm that has no such form throws.
     virtual AddendTransform as_transform(float factor) const;
+    // The norm's weight and eps, if it is x * rsqrt(mean(x^2) + eps) * weight over the row and nothing else.
+    virtual bool plain_rms(const float** weight, float* eps) const { return false; }
     // The float32 rows x [n, width] normed in place (no addend, no cast): for an embedding that is normed before it
     // becomes the residual stream.  A norm that has no such form throws.
     virtual void apply_in_place(Tensor& x, StepContext& ctx, int n);
@@ -411,6 +426,7 @@ public:
     // True: in this step the mixer applies ctx.row_scale to what its first product gives, so the norm in front may
     // leave the row's factor out (see RowScale).  A mixer that says nothing always gets finished rows.
     virtual bool takes_unscaled_rows(const StepContext&) const { return false; }
+    virtual bool decode_layer(DecodeLayerSpec&) const { return false; }              // see DecodeLayerSpec
 };
 
 class QE_API FeedForward : public Part {
@@ -418,6 +434,7 @@ public:
     using Part::Part;
     virtual Addend forward(const Tensor& x, StepContext& ctx) = 0;
     virtual bool takes_unscaled_rows(const StepContext&) const { return false; }     // as Mixer's
+    virtual bool decode_layer(DecodeLayerSpec&) const { return false; }
 };
 
 class QE_API Embedding : public Part {
@@ -442,6 +459,8 @@ public:
     // The offer of the layer's first norm, if in this step it would take rows prepared by the layer in front (the
     // model hands it to that layer as ctx.next_layer_norm).
     virtual NormAhead first_norm(const StepContext&) const { return NormAhead(); }
+    // The whole layer for the one-launch decode step; false: it does not fit.
+    virtual bool decode_layer(DecodeLayerSpec&) const { return false; }
 };
 
 // ---- registries -------------------------------------------------------------------------------------------------------

@@ -1,0 +1,94 @@
+"""All layers of a decode step in one launch (csrc/decode_layers.cu), at the sizes where it can go wrong: against float64 and
+against the same step with a launch per operation."""
+import tempfile
+
+import numpy as np
+import pytest
+
+from helpers import make_model, random_tokens
+
+pytestmark = pytest.mark.gpu
+
+INIT = dict(seed=5, std=0.04, scale_low=0.8, scale_high=1.2)
+
+
+def _config(width, inner, heads, kv_heads, layers, vocab=640):
+    return dict(architectures=["Qwen3ForCausalLM"], num_hidden_layers=layers, hidden_size=width, intermediate_size=inner,
+                num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=128, vocab_size=vocab, max_position_embeddings=2048,
+                rope_theta=1e6, rms_norm_eps=1e-6, tie_word_embeddings=False, attention_bias=False)
+
+
+def _steps(folder, page_size, toks, prefixes, steps, options, graphs=True):
+    """Logits of every decoded token, [steps, rows, vocab], and whether the last step was a replay."""
+    from purhie_b200.engine import Engine, StepEntry
+    eng = Engine.from_folder(folder, dtype="bfloat16", page_size=page_size, max_tokens=8192, max_requests=len(prefixes), poison_cache=True,
+                             cuda_graphs=graphs, step_options=options)
+    out = []
+    for r, n in enumerate(prefixes):
+        eng.add_request(r)
+        if n:
+            eng.step([StepEntry(r, toks[r][:n], [])])
+    for k in range(steps):
+        out.append(eng.step([StepEntry(r, toks[r][n + k:n + k + 1], [0]) for r, n in enumerate(prefixes)]).copy())
+    replayed = eng.last_stats.replayed_graph
+    eng.close()
+    return np.stack(out), replayed
+
+
+# width, inner, heads, kv heads, layers, page size, tokens in the cache per row
+CASES = [
+    (64, 64, 1, 1, 1, 16, [0]),                                   # one group of 16 rows per product and less, nothing cached
+    (192, 320, 8, 1, 2, 8, [31]),                                 # K of part of a stage, one pair for all CTAs, a block's last slot
+    (320, 1088, 4, 2, 3, 16, [32, 1, 700]),                       # ragged K, a new block, lengths that differ
+    (1024, 3072, 16, 8, 2, 32, [63, 64, 65, 200, 17, 16, 15, 2]), # eight rows, pages of a whole block
+    (512, 4672, 6, 6, 2, 16, [5, 1500, 33, 0, 31, 32, 90, 1]),    # K in chunks through half of the places, with a ragged last one
+    (2048, 6144, 8, 8, 2, 16, [1900]),                            # one row whose keys many CTAs share
+    (1024, 17408, 8, 4, 1, 16, [40]),                             # one row, K longer than all places
+]
+
+
+@pytest.mark.parametrize("width,inner,heads,kv_heads,layers,page_size,prefixes", CASES)
+def test_one_launch_gives_the_layers(width, inner, heads, kv_heads, layers, page_size, prefixes):
+    from plain import qwen3_plain as P
+    steps = 4
+    with tempfile.TemporaryDirectory() as tmp:
+        cfg = make_model(tmp, _config(width, inner, heads, kv_heads, layers), INIT, "bfloat16")
+        pc, pw = P.read_model(tmp)
+        toks = [random_tokens(n + steps, cfg.vocab_size, 11 + r) for r, n in enumerate(prefixes)]
+        exact = np.stack([P.forward(pc, pw, t)[n:].numpy() for t, n in zip(toks, prefixes)], axis=1)
+        one, replayed = _steps(tmp, page_size, toks, prefixes, steps, None)
+        again, _ = _steps(tmp, page_size, toks, prefixes, steps, None, graphs=False)
+        many, _ = _steps(tmp, page_size, toks, prefixes, steps, {"decode_stack": "off"})
+    assert replayed
+    assert np.array_equal(one, again)                             # nothing depends on the order in which CTAs arrive
+    error = lambda got: np.linalg.norm((got - exact).ravel()) / np.linalg.norm(exact.ravel())
+    # both forms round the same quantities to bfloat16 in the same places (normed rows, q, k, v, probabilities, heads,
+    # activations) and add in float32: errors of one distribution, a quarter apart at most at these few thousand logits
+    assert error(one) <= 1.25 * error(many), (error(one), error(many))
+    assert error(one) < 0.02
+
+
+def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
+    """Nine rows, a portion beside a decoded token, and a step with a kernel choice are made of a launch per operation."""
+    from purhie_b200 import native
+    from purhie_b200.engine import Engine, StepEntry
+    config = _config(256, 512, 4, 2, 3)
+    toks = random_tokens(64, config["vocab_size"], 3)
+
+    def launches(rows, portion, options):
+        eng = Engine.from_random(config, 3, dtype="bfloat16", max_tokens=4096, max_requests=10, cuda_graphs=False, step_options=options)
+        for r in range(rows):
+            eng.add_request(r)
+            eng.step([StepEntry(r, toks[:20], [])])
+        entries = [StepEntry(r, toks[20:21], []) for r in range(rows)]
+        if portion:
+            eng.add_request("p")
+            entries.append(StepEntry("p", toks[:5], []))
+        before = native.lib().qe_launches()
+        eng.step(entries)
+        n = native.lib().qe_launches() - before
+        eng.close()
+        return n
+    assert launches(1, False, None) == launches(8, False, None) == 2          # the embedding, the layers
+    for rows, portion, options in [(9, False, None), (3, True, None), (3, False, {"decode_kernel": "cp_async"}), (3, False, {"decode_stack": "off"})]:
+        assert launches(rows, portion, options) > 3 * config["num_hidden_layers"]
