@@ -97,9 +97,6 @@ __device__ __forceinline__ int add_acq_rel(int32_t* p, int v) {
 }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS) : "memory"); }
-__device__ __forceinline__ void arrive_n(uint64_t* bar, uint32_t n) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(mb::smem_addr(bar)), "r"(n) : "memory");
-}
 __device__ __forceinline__ void load_weights(void* dst, const CUtensorMap* map, uint64_t* bar, int row, int block) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(block) : "memory");
@@ -329,11 +326,17 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
     float* red = (float*)c.x;                                            // [warps][G][D + 2]: the activations' place is free here
     float* mine = red + (size_t)warp * G * RS;
     const int r0 = lane >> 2;
-    wait_for(c.ready, ready, c, error, PH_ERR_WAIT_LAYERS_DATA);
-    ready ^= 1;
     Piece s;
     for (int i = 0; piece_at(c, p, i, s); ++i) {
         const int z = c.z[s.row], pair = s.row * HKV + s.head;
+        // (the rotation does not wait for the product in front)
+        const int pos = min(max(p.a.rotation_positions[s.row], 0), p.a.max_position - 1);
+        const float4* cs = (const float4*)(p.a.rotation + (size_t)pos * D) + (lane & 15);
+        const float4 co = cs[0], si = cs[16];
+        if (!i) {
+            wait_for(c.ready, ready, c, error, PH_ERR_WAIT_LAYERS_DATA);
+            ready ^= 1;
+        }
         const bool tail = s.b0 + s.n == s.blocks;
         // the group's queries, normed and rotated, and with the last block the step's own key and value
         for (int task = warp; task < G + (tail ? 2 : 0); task += WARPS) {
@@ -344,9 +347,6 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
                 const float ss = warp_sum(fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))));
                 const float inv = rsqrtf(ss / (float)D + p.a.qk_eps);
                 v.x *= inv * w.x; v.y *= inv * w.y; v.z *= inv * w.z; v.w *= inv * w.w;
-                const int pos = min(max(p.a.rotation_positions[s.row], 0), p.a.max_position - 1);
-                const float4* cs = (const float4*)(p.a.rotation + (size_t)pos * D) + (lane & 15);
-                const float4 co = cs[0], si = cs[16];
                 float4 o;
                 o.x = __shfl_xor_sync(0xffffffffu, v.x, 16); o.y = __shfl_xor_sync(0xffffffffu, v.y, 16);
                 o.z = __shfl_xor_sync(0xffffffffu, v.z, 16); o.w = __shfl_xor_sync(0xffffffffu, v.w, 16);
@@ -378,10 +378,15 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
         for (int dt = 0; dt < D / 8; ++dt)
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[dt][i] = 0.0f;
-        // four blocks at a time, two warps a block, 16 keys each
+        // Four blocks at a time, two warps a block, 16 keys each.  Every warp sees every stage and answers for it: a warp that
+        // passed over stages could ask for one whose fill before the last has the parity it waits for.
         for (int j = 0; j < s.n; ++j, ring.next(p.stages)) {
-            if ((j & 3) != (warp >> 1)) continue;
             wait_for(&c.full[ring.stage], ring.phase, c, error, PH_ERR_WAIT_LAYERS_DATA);
+            if ((j & 3) != (warp >> 1)) {
+                __syncwarp();
+                if (lane == 0) mb::arrive(&c.empty[ring.stage]);
+                continue;
+            }
             unsigned char* st_ptr = c.ring + ring.stage * STAGE;
             const uint32_t st = smem_u32(st_ptr);
             const int k0 = (warp & 1) * 16, key0 = (s.b0 + j) * KEYS + k0;
@@ -423,7 +428,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
                 if (edge) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // our stores, before the next copy lands there
             }
             __syncwarp();
-            if (lane == 0) arrive_n(&c.empty[ring.stage], WARPS / 2);    // two warps answer for eight
+            if (lane == 0) mb::arrive(&c.empty[ring.stage]);
         }
         // merge the eight warps (a group has at most eight heads: fragment rows 8 .. 15 are padding)
         if (r0 < G) {
@@ -500,7 +505,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
 
 __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params p) {
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // (an offset: the compiler still sees shared memory)
     const int M = p.a.rows, E = p.a.width, HKV = p.a.kv_heads;
     const int CTAS = gridDim.x;
     Cta c;
