@@ -595,53 +595,67 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
 
     if (warp == WARPS) {
         // ---- the ring: weights and cached keys in the order of their use, whatever the other CTAs are at ----
-        Ring ring;
-        int filled = 0;
-        auto fill = [&](uint32_t bytes) {                                // a free stage, with so many bytes announced
-            if (lane == 0) {
-                wait_for(&c.empty[ring.stage], ring.phase ^ 1, c, error, PH_ERR_WAIT_LAYERS_RING);
-                if (!*c.dead) mb::arrive_expect_tx(&c.full[ring.stage], bytes);
-            }
-            return __shfl_sync(0xffffffffu, lane == 0 ? *c.dead : 0, 0) == 0;
-        };
-        auto weights = [&](const CUtensorMap* map, int which) {
-            const int K = widths[which], nseg = segments(K), cs = chunk_of(nseg, p.slots);
-            for (int c0 = 0; c0 < nseg; c0 += cs)
-                for (int gi = 0; gi < c.ng[which]; ++gi)
-                    for (int seg = c0; seg < min(c0 + cs, nseg); ++seg) {
-                        if (!fill(STAGE)) return false;                  // (K's end counts in full: zeros)
-                        if (lane == 0) load_weights(c.ring + ring.stage * STAGE, map, &c.full[ring.stage], (c.g0[which] + gi) * 16, seg * (SEG / 64));
-                        ring.next(p.stages);
-                        ++filled;
-                    }
-            return true;
-        };
-        auto keys = [&](const CUtensorMap* map) {
-            int at = 0;
-            Piece s;
-            for (int n = 0; piece_at(c, p, n, s); ++n)
-                for (int j = 0; j < s.n; ++j, at += ppb) {
-                    if (!fill(KEYS * D * 4)) return false;
-                    if (lane < ppb) {
-                        const int row = at + lane < PAGES ? c.pages[at + lane] : page_row(c, p, s.row, s.head, s.b0 + j, lane);
-                        load_page(c.ring + ring.stage * STAGE + lane * p.a.page_size * 512, map, &c.full[ring.stage], row);
-                    }
-                    ring.next(p.stages);
-                    ++filled;
+        // One thread, with as little as possible between two copies: a stage's time is the longer of its bytes' and of this
+        // loop's turn.
+        if (lane == 0) {
+            Ring ring;
+            int filled = 0;
+            unsigned char* to = c.ring;
+            auto fill = [&](uint32_t bytes) {                            // a free stage, with so many bytes announced
+                if (!mb::try_wait(&c.empty[ring.stage], ring.phase ^ 1)) {
+                    wait_for(&c.empty[ring.stage], ring.phase ^ 1, c, error, PH_ERR_WAIT_LAYERS_RING);
+                    if (*c.dead) return false;
                 }
-            return true;
-        };
-        const CUtensorMap* maps = (const CUtensorMap*)p.a.maps;
-        for (int l = 0; l < p.a.n_layers; ++l, maps += MAPS) {
-            if (lane < 2 * MAPS && (lane < MAPS ? l == 0 : l + 1 < p.a.n_layers)) asm volatile("prefetch.tensormap [%0];" ::"l"(maps + lane) : "memory");
-            if (!weights(maps, 0) || !keys(maps + 4) || !weights(maps + 1, 1) || !weights(maps + 2, 2) || !weights(maps + 3, 3)) break;
-        }
-        if (*c.dead && lane == 0) {
-            // consumers no longer wait for what is on its way: do not leave before it has landed
-            for (int i = min(filled, p.stages); i; --i) {
-                if (ring.stage == 0) { ring.stage = p.stages; ring.phase ^= 1; }
-                --ring.stage;
-                mb::wait(&c.full[ring.stage], ring.phase, error, PH_ERR_WAIT_LAYERS_RING);
+                mb::arrive_expect_tx(&c.full[ring.stage], bytes);
+                return true;
+            };
+            auto filled_one = [&] {
+                ++filled;
+                to += STAGE;
+                if (++ring.stage == p.stages) { ring.stage = 0; ring.phase ^= 1; to = c.ring; }
+            };
+            auto weights = [&](const CUtensorMap* map, int g0, int ng, int K) {
+                const int nseg = segments(K), cs = chunk_of(nseg, p.slots);
+                for (int c0 = 0; c0 < nseg; c0 += cs) {
+                    const int end = min(c0 + cs, nseg) * (SEG / 64);
+                    for (int row = g0 * 16; row < (g0 + ng) * 16; row += 16)
+                        for (int block = c0 * (SEG / 64); block < end; block += SEG / 64) {
+                            if (!fill(STAGE)) return false;              // (K's end counts in full: zeros)
+                            load_weights(to, map, &c.full[ring.stage], row, block);
+                            filled_one();
+                        }
+                }
+                return true;
+            };
+            auto keys = [&](const CUtensorMap* map) {
+                int at = 0;
+                Piece s;
+                for (int n = 0; piece_at(c, p, n, s); ++n)
+                    for (int j = 0; j < s.n; ++j) {
+                        if (!fill(KEYS * D * 4)) return false;
+                        for (int i = 0; i < ppb; ++i, ++at)
+                            load_page(to + i * p.a.page_size * 512, map, &c.full[ring.stage],
+                                      at < PAGES ? c.pages[at] : page_row(c, p, s.row, s.head, s.b0 + j, i));
+                        filled_one();
+                    }
+                return true;
+            };
+            const CUtensorMap* maps = (const CUtensorMap*)p.a.maps;
+            for (int i = 0; i < MAPS; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(maps + i) : "memory");
+            for (int l = 0; l < p.a.n_layers; ++l, maps += MAPS) {
+                if (l + 1 < p.a.n_layers)
+                    for (int i = 0; i < MAPS; ++i) asm volatile("prefetch.tensormap [%0];" ::"l"(maps + MAPS + i) : "memory");
+                if (!weights(maps, c.g0[0], c.ng[0], widths[0]) || !keys(maps + 4) || !weights(maps + 1, c.g0[1], c.ng[1], widths[1]) ||
+                    !weights(maps + 2, c.g0[2], c.ng[2], widths[2]) || !weights(maps + 3, c.g0[3], c.ng[3], widths[3]))
+                    break;
+            }
+            if (*c.dead) {
+                // consumers no longer wait for what is on its way: do not leave before it has landed
+                for (int i = min(filled, p.stages); i; --i) {
+                    if (ring.stage == 0) { ring.stage = p.stages; ring.phase ^= 1; }
+                    --ring.stage;
+                    mb::wait(&c.full[ring.stage], ring.phase, error, PH_ERR_WAIT_LAYERS_RING);
+                }
             }
         }
     } else if (warp == WARPS + 1) {

@@ -69,13 +69,14 @@ def test_one_launch_gives_the_layers(width, inner, heads, kv_heads, layers, page
 
 
 def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
-    """Nine rows, a portion beside a decoded token, and a step with a kernel choice are made of a launch per operation."""
+    """Nine rows, a portion beside a decoded token, a step with a kernel choice and a width that divides badly are made of a launch
+    per operation."""
     from purhie_b200 import native
     from purhie_b200.engine import Engine, StepEntry
     config = _config(256, 512, 4, 2, 3)
     toks = random_tokens(64, config["vocab_size"], 3)
 
-    def launches(rows, portion, options):
+    def launches(rows, portion, options, config=config):
         eng = Engine.from_random(config, 3, dtype="bfloat16", max_tokens=4096, max_requests=10, cuda_graphs=False, step_options=options)
         for r in range(rows):
             eng.add_request(r)
@@ -92,3 +93,5 @@ def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
     assert launches(1, False, None) == launches(8, False, None) == 2          # the embedding, the layers
     for rows, portion, options in [(9, False, None), (3, True, None), (3, False, {"decode_kernel": "cp_async"}), (3, False, {"decode_stack": "off"})]:
         assert launches(rows, portion, options) > 3 * config["num_hidden_layers"]
+    # 160 groups of 16 rows for 148 CTAs, twice a layer: the largest shares lose what the launches cost
+    assert launches(1, False, None, _config(2560, 9728, 32, 8, 1)) > 3
