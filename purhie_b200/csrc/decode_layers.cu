@@ -12,8 +12,9 @@
 //
 // Products: groups of 16 output rows are dealt to the CTAs so that every CTA streams the same bytes per layer (`shares`); K
 // stays whole in a CTA, so a result is written once, by one CTA, and nothing is added up between CTAs.  A stage is 16 weight
-// rows x 512 of K, one box of eight blocks of 64, 128-byte swizzled.  Eight warps take 64 of the 512 each on
-// mma.sync.m16n8k16 with the weights as the 16 rows and the tokens as the 8 columns: the work is a stream from memory (8 rows:
+// rows x 512 of K, one box of eight blocks of 64, 128-byte swizzled (as 16 copies of 1 KB the same bytes came at 2.6 TB/s, the copy
+// engine bound by their number; as a box with the rows outermost two rows meet in a bank: 8B shape 85.7 us).  Eight warps take
+// 64 of the 512 each on mma.sync.m16n8k16 with the weights as the 16 rows and the tokens as the 8 columns: the work is a stream from memory (8 rows:
 // 16 flops a byte), and this instruction takes both operands from registers as 16-byte reads deliver them, where a
 // tensor-memory accumulator would add its own round trip to each of 5 parts.  The eight partial sums are added in ascending
 // order of K.
@@ -23,11 +24,11 @@
 // as one box per page as in attention_decode_bulk.cu; the step's own key and value are made by the CTA that holds the pair's last
 // block, which writes them to the cache and over their row of the stage.
 //
-// Measured (us a layer, a launch per operation -> this): 0.6B shape behind 2,048 tokens 38.8 -> 29.3 at one row, 51.0 -> 41.7 at eight;
-// width 2,048 51.4 -> 42.3 and 65.1 -> 57.1; 8B shape 90.2 -> 86.5 and 104.4 -> 101.9.  What bounds a layer now is the way of a
+// Measured (us a layer behind 2,048 tokens, a launch per operation -> this): 0.6B shape 38.8 -> 28.1 at one row, 51.0 -> 40.6 at eight;
+// width 2,048 51.4 -> 39.5 and 65.1 -> 54.5; 8B shape 90.2 -> 84.2 and 104.4 -> 100.3.  What bounds a layer now is the way of a
 // result to the other CTAs, five times: barrier and release 1.2 us, the poll 0.7, the rows' way to shared memory 1.2, and in the
-// attention twice that for the merge.
-
+// attention twice that for the merge; with larger weights also the copying thread's turn (a stage in 390 ns, 42 GB/s an SM).
+//
 // Waiting: results pass between CTAs through global memory behind counters (release adds, acquire polls), which is safe
 // because the launch is cooperative: all CTAs are resident.  Every wait is bounded; one that runs out reports through the error
 // word and lets its CTA run on without waiting, so that no other CTA is held up and the launch ends.
