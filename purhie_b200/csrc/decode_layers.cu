@@ -98,6 +98,10 @@ __device__ __forceinline__ int add_acq_rel(int32_t* p, int v) {
 }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS) : "memory"); }
+// A copy from the host wrote the map, which the copy engine reads through a proxy and cache of its own: nothing else orders the two.
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void load_weights(void* dst, const CUtensorMap* map, uint64_t* bar, int row, int block) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(block) : "memory");
@@ -534,6 +538,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < p.a.n_layers * (int)(sizeof(PhDecodeLayer) / 8); i += NTHREADS)
         ((uint64_t*)c.layers)[i] = ((const uint64_t*)p.a.layers)[i];
+    // (an engine's maps may lie where those of a closed one lay; a map a thread, in front of the barriers before the first copy)
+    for (int i = threadIdx.x; i < p.a.n_layers * MAPS; i += NTHREADS) acquire_map((const CUtensorMap*)p.a.maps + i);
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) { mb::init(&c.full[s], 1); mb::init(&c.empty[s], WARPS); }
         for (int s = 0; s < p.slots; ++s) mb::init(&c.x_full[s], 1);

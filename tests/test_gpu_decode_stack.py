@@ -95,3 +95,22 @@ def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
         assert launches(rows, portion, options) > 3 * config["num_hidden_layers"]
     # 160 groups of 16 rows for 148 CTAs, twice a layer: the largest shares lose what the launches cost
     assert launches(1, False, None, _config(2560, 9728, 32, 8, 1)) > 3
+
+
+def test_engines_one_after_the_other_read_their_own_weights_and_caches():
+    """Engines of other weights and page sizes whose descriptors may lie where a closed engine's lay."""
+    from purhie_b200.engine import Engine, StepEntry
+    config = _config(256, 512, 4, 2, 3)
+    toks = random_tokens(64, config["vocab_size"], 3)
+
+    def logits(seed, page_size, options):
+        eng = Engine.from_random(config, seed, dtype="bfloat16", page_size=page_size, max_tokens=1024, max_requests=1, step_options=options)
+        eng.add_request(0)
+        eng.step([StepEntry(0, toks[:40], [])])
+        out = np.stack([eng.step([StepEntry(0, toks[40 + k:41 + k], [0])]).copy() for k in range(3)])
+        eng.close()
+        return out
+    # two roundings of a few dozen quantities to bfloat16 (2^-9 each) in three layers; another engine's weights differ by more than 1
+    for i in range(6):
+        one, many = logits(i, 8 << i % 3, None), logits(i, 8 << i % 3, {"decode_stack": "off"})
+        assert np.linalg.norm(one - many) < 0.03 * np.linalg.norm(many)
