@@ -314,6 +314,10 @@ API int qe_engine_set_error_word(inference_model_t* m, int which, int code) {
         return 0;
     });
 }
+// Make the next one-launch decode step run out of a wait after so many cycles (0: waits as usual again).
+API int qe_engine_stall_decode_stack(inference_model_t* m, long long wait_cycles) {
+    return guarded([&] { return need_engine(m).stall_decode_stack(wait_cycles) ? 0 : -1; });
+}
 // ---- timing on the device, for the benchmark ---------------------------------------------------------------------------
 // `warmup + steps` decode steps of n requests (live, each with its prefix in the cache): step k feeds request i the
 // token tokens[i * (warmup + steps) + k] from the host, and, with `sample`, every step's logits go through the greedy

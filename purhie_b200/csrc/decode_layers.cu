@@ -31,7 +31,8 @@
 //
 // Waiting: results pass between CTAs through global memory behind counters (release adds, acquire polls), which is safe
 // because the launch is cooperative: all CTAs are resident.  Every wait is bounded; one that runs out reports through the error
-// word and lets its CTA run on without waiting, so that no other CTA is held up and the launch ends.
+// word, and its CTA's threads run on without waiting as they notice, so that no other CTA is held up and the launch ends.  Such a
+// thread frees no place of a ring any more (nothing is asked for twice over), and a CTA leaves when all that it asked for has landed.
 #include "attention_mma.cuh"
 #include "decode_layers.h"
 #include "mbarrier.cuh"
@@ -79,6 +80,7 @@ struct Params {
     int stages, slots, acc_groups, x_bytes, page_shift;
     long long rows_per_page;
     float scale_log2;
+    long long wait_cycles;
 };
 
 __host__ __device__ inline int segments(int k) { return (k + SEG - 1) / SEG; }
@@ -135,6 +137,7 @@ struct Cta {
     PhDecodeLayer* layers;
     uint64_t *full, *empty, *x_full, *x_empty, *ready;
     volatile int* dead;                         // a wait ran out: nobody waits any more
+    mutable bool gone;                          // ... and this thread knows: it neither waits nor frees places
     int* flag;
     int g0[4], ng[4];                           // this CTA's groups in each product
     int sharers;                                // CTAs that have a piece of the attention (0: more pairs than CTAs)
@@ -142,27 +145,35 @@ struct Cta {
 };
 
 // Looks again and again, the first few hundred times without a look at the clock; gives up for the whole CTA when the limit
-// passes (4e9 cycles: two seconds at the highest clock).
+// passes (4e9 cycles: two seconds at the highest clock).  False: nobody waits any more.
 constexpr long long WAIT_CYCLES = 4000000000ll;
-template <typename Done> __device__ __forceinline__ void wait_until(Done done, const Cta& c, int* error, int code) {
+template <typename Done> __device__ __forceinline__ bool wait_until(Done done, const Cta& c, const Params& p, int code) {
+    if (c.gone) return false;
     long long t0 = 0;
     for (uint32_t i = 1; !done(); ++i) {
         if (i & 255u) continue;
-        if (*c.dead) return;
-        const long long now = clock64();
-        if (i == 256u) t0 = now;
-        else if (now - t0 > WAIT_CYCLES) {
-            atomicExch(error, code);
+        if (!*c.dead) {
+            const long long now = clock64();
+            if (i == 256u) t0 = now;
+            if (now - t0 <= p.wait_cycles) continue;
+            atomicExch(p.a.error_flag, code);
             *c.dead = 1;
-            return;
         }
+        c.gone = true;
+        return false;
     }
+    return true;
 }
-__device__ __forceinline__ void wait_for(uint64_t* bar, uint32_t parity, const Cta& c, int* error, int code) {
-    wait_until([&] { return mb::try_wait(bar, parity); }, c, error, code);
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, const Cta& c, const Params& p, int code) {
+    return wait_until([&] { return mb::try_wait(bar, parity); }, c, p, code);
 }
-__device__ __forceinline__ void wait_count(const int32_t* p, int target, const Cta& c, int* error) {
-    wait_until([&] { return load_acquire(p) >= target; }, c, error, PH_ERR_WAIT_LAYERS_PEERS);
+__device__ __forceinline__ bool wait_count(const int32_t* counter, int target, const Cta& c, const Params& p) {
+    return wait_until([&] { return load_acquire(counter) >= target; }, c, p, PH_ERR_WAIT_LAYERS_PEERS);
+}
+// A warp's answer for a place that it has read.
+__device__ __forceinline__ void free_place(uint64_t* bar, const Cta& c) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0 && !c.gone) mb::arrive(bar);
 }
 
 // The results that this part wrote are complete: every consumer's stores, then one add.
@@ -220,8 +231,7 @@ __device__ __forceinline__ void product(const Cta& c, const Params& p, Ring& rin
     if (!ng) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int M = p.a.rows, E = p.a.width;
-    int* error = p.a.error_flag;
-    wait_for(c.ready, ready, c, error, PH_ERR_WAIT_LAYERS_DATA);
+    wait_for(c.ready, ready, c, p, PH_ERR_WAIT_LAYERS_DATA);
     ready ^= 1;
     if (KIND != RESIDUAL && warp < M) {
         float s = 0.0f;
@@ -254,8 +264,8 @@ __device__ __forceinline__ void product(const Cta& c, const Params& p, Ring& rin
             float s[2][4] = {};
             for (int seg = c0; seg < c1; ++seg) {
                 const int slot = whole ? seg : half * cs + seg - c0;
-                wait_for(&c.full[ring.stage], ring.phase, c, error, PH_ERR_WAIT_LAYERS_DATA);
-                if (gi == 0) wait_for(&c.x_full[slot], (x_parity >> slot) & 1u, c, error, PH_ERR_WAIT_LAYERS_DATA);
+                wait_for(&c.full[ring.stage], ring.phase, c, p, PH_ERR_WAIT_LAYERS_DATA);
+                if (gi == 0) wait_for(&c.x_full[slot], (x_parity >> slot) & 1u, c, p, PH_ERR_WAIT_LAYERS_DATA);
                 if (seg * SEG + warp * 64 < K) {
                     const unsigned char* w = c.ring + ring.stage * STAGE + w_off;
                     const unsigned char* x = c.x + slot * slot_bytes + x_off;
@@ -267,8 +277,7 @@ __device__ __forceinline__ void product(const Cta& c, const Params& p, Ring& rin
                         mma_bf16(s[h], a.z, b.z, a.w, b.w, v.z, v.w);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mb::arrive(&c.empty[ring.stage]);
+                free_place(&c.empty[ring.stage], c);
                 ring.next(p.stages);
             }
             float* red = c.red + (unit & 1) * (WARPS * ROWS * RED);
@@ -310,11 +319,8 @@ __device__ __forceinline__ void product(const Cta& c, const Params& p, Ring& rin
         // the places of this chunk are free
         const uint32_t used = (c1 - c0 == 32 ? 0xffffffffu : ((1u << (c1 - c0)) - 1u)) << (whole ? 0 : half * cs);
         x_parity ^= used;
-        __syncwarp();
-        if (lane == 0) {
-            if (whole) { mb::arrive(&c.x_empty[0]); mb::arrive(&c.x_empty[1]); }
-            else mb::arrive(&c.x_empty[half]);
-        }
+        if (whole || half == 0) free_place(&c.x_empty[0], c);
+        if (whole || half == 1) free_place(&c.x_empty[1], c);
     }
 }
 
@@ -327,7 +333,6 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
     const int width = (HQ + 2 * HKV) * D;
     const int ps = p.a.page_size, psh = p.page_shift;
     constexpr int RS = D + 2;
-    int* error = p.a.error_flag;
     float* red = (float*)c.x;                                            // [warps][G][D + 2]: the activations' place is free here
     float* mine = red + (size_t)warp * G * RS;
     const int r0 = lane >> 2;
@@ -339,7 +344,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
         const float4* cs = (const float4*)(p.a.rotation + (size_t)pos * D) + (lane & 15);
         const float4 co = cs[0], si = cs[16];
         if (!i) {
-            wait_for(c.ready, ready, c, error, PH_ERR_WAIT_LAYERS_DATA);
+            wait_for(c.ready, ready, c, p, PH_ERR_WAIT_LAYERS_DATA);
             ready ^= 1;
         }
         const bool tail = s.b0 + s.n == s.blocks;
@@ -386,10 +391,9 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
         // Four blocks at a time, two warps a block, 16 keys each.  Every warp sees every stage and answers for it: a warp that
         // passed over stages could ask for one whose fill before the last has the parity it waits for.
         for (int j = 0; j < s.n; ++j, ring.next(p.stages)) {
-            wait_for(&c.full[ring.stage], ring.phase, c, error, PH_ERR_WAIT_LAYERS_DATA);
+            wait_for(&c.full[ring.stage], ring.phase, c, p, PH_ERR_WAIT_LAYERS_DATA);
             if ((j & 3) != (warp >> 1)) {
-                __syncwarp();
-                if (lane == 0) mb::arrive(&c.empty[ring.stage]);
+                free_place(&c.empty[ring.stage], c);
                 continue;
             }
             unsigned char* st_ptr = c.ring + ring.stage * STAGE;
@@ -432,8 +436,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
                 }
                 if (edge) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // our stores, before the next copy lands there
             }
-            __syncwarp();
-            if (lane == 0) mb::arrive(&c.empty[ring.stage]);
+            free_place(&c.empty[ring.stage], c);
         }
         // merge the eight warps (a group has at most eight heads: fragment rows 8 .. 15 are padding)
         if (r0 < G) {
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
     const int M = p.a.rows, E = p.a.width, HKV = p.a.kv_heads;
     const int CTAS = gridDim.x;
     Cta c;
+    c.gone = false;
     c.ring = smem;
     c.x = c.ring + p.stages * STAGE;
     c.red = (float*)(c.x + p.x_bytes);
@@ -597,7 +601,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
 
     int32_t* counters = p.a.counters + 1;                                // [0]: CTAs that are done
     int32_t* pairs = counters + 1 + PARTS * p.a.n_layers;
-    int* error = p.a.error_flag;
     const int widths[4] = {E, p.a.heads * D, E, p.a.inner};
 
     if (warp == WARPS) {
@@ -609,10 +612,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
             int filled = 0;
             unsigned char* to = c.ring;
             auto fill = [&](uint32_t bytes) {                            // a free stage, with so many bytes announced
-                if (!mb::try_wait(&c.empty[ring.stage], ring.phase ^ 1)) {
-                    wait_for(&c.empty[ring.stage], ring.phase ^ 1, c, error, PH_ERR_WAIT_LAYERS_RING);
-                    if (*c.dead) return false;
-                }
+                if (!mb::try_wait(&c.empty[ring.stage], ring.phase ^ 1) &&
+                    !wait_for(&c.empty[ring.stage], ring.phase ^ 1, c, p, PH_ERR_WAIT_LAYERS_RING))
+                    return false;
                 mb::arrive_expect_tx(&c.full[ring.stage], bytes);
                 return true;
             };
@@ -656,13 +658,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
                     !weights(maps + 2, c.g0[2], c.ng[2], widths[2]) || !weights(maps + 3, c.g0[3], c.ng[3], widths[3]))
                     break;
             }
-            if (*c.dead) {
-                // consumers no longer wait for what is on its way: do not leave before it has landed
-                for (int i = min(filled, p.stages); i; --i) {
-                    if (ring.stage == 0) { ring.stage = p.stages; ring.phase ^= 1; }
-                    --ring.stage;
-                    mb::wait(&c.full[ring.stage], ring.phase, error, PH_ERR_WAIT_LAYERS_RING);
-                }
+            // do not leave before the last of it has landed: consumers that are gone do not wait for it
+            for (int i = min(filled, p.stages); i; --i) {
+                if (ring.stage == 0) { ring.stage = p.stages; ring.phase ^= 1; }
+                --ring.stage;
+                mb::wait(&c.full[ring.stage], ring.phase, p.a.error_flag, PH_ERR_WAIT_LAYERS_RING);
             }
         }
     } else if (warp == WARPS + 1) {
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
         bool ok = true;
         auto alive = [&] { return __shfl_sync(0xffffffffu, lane == 0 ? *c.dead : 0, 0) == 0; };
         auto begin = [&](const int32_t* counter, int target) {           // every lane looks, so every lane may go on
-            wait_count(counter, target, c, error);
+            wait_count(counter, target, c, p);
             fence_async();
             if (lane == 0) mb::arrive(c.ready);
             ok = alive();
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
         auto make_room = [&](bool whole, int half, int slot0, int c0, int n, int K) {
             for (int h = 0; h < 2; ++h)
                 if (whole || h == half) {
-                    wait_for(&c.x_empty[h], x_free[h], c, error, PH_ERR_WAIT_LAYERS_RING);
+                    wait_for(&c.x_empty[h], x_free[h], c, p, PH_ERR_WAIT_LAYERS_RING);
                     x_free[h] ^= 1;
                 }
             ok = alive();
@@ -713,9 +713,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
             if (ok && c.ng[2]) load(k + 3, CTAS, p.a.xw, E);
             if (ok && c.ng[3]) load(k + 4, CTAS, p.a.act, widths[3]);
         }
-        if (*c.dead && lane == 0)
+        if (lane == 0)                                                   // (as the ring's thread)
             for (int s = 0; s < p.slots; ++s)
-                if ((pending >> s) & 1u) mb::wait(&c.x_full[s], ((x_parity >> s) & 1u) ^ 1u, error, PH_ERR_WAIT_LAYERS_RING);
+                if ((pending >> s) & 1u) mb::wait(&c.x_full[s], ((x_parity >> s) & 1u) ^ 1u, p.a.error_flag, PH_ERR_WAIT_LAYERS_RING);
     } else {
         // ---- the work ----
         Ring ring;
@@ -896,6 +896,7 @@ PH_EXPORT int ph_decode_layers(const PhDecodeLayersArgs* args, cudaStream_t stre
     p.page_shift = a.page_size == 8 ? 3 : a.page_size == 16 ? 4 : 5;
     p.rows_per_page = a.page_stride / D;
     p.scale_log2 = a.scale * LOG2E;
+    p.wait_cycles = a.wait_cycles > 0 ? a.wait_cycles : WAIT_CYCLES;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

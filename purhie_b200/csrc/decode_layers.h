@@ -44,4 +44,5 @@ struct PhDecodeLayersArgs {
     float* part_o;                     // [CTAs][HQ / HKV][128]
     float* part_ml;                    // [CTAs][HQ / HKV][2]
     int* error_flag;
+    long long wait_cycles;             // limit of every wait (0: two seconds)
 };

@@ -520,6 +520,11 @@ void Engine::inject_error_word(int which, int code) {
     QE_CUDA(cudaStreamSynchronize(stream_));
 }
 
+bool Engine::stall_decode_stack(long long wait_cycles) {
+    if (decode_stack_) decode_stack_->stall(wait_cycles, stream_);
+    return decode_stack_ != nullptr;
+}
+
 void Engine::read_logits(const Tensor& logits, float* host) {
     if (!logits.defined()) return;
     QE_CUDA(cudaMemcpyAsync(host, logits.data, logits.bytes(), cudaMemcpyDeviceToHost, stream_));

@@ -139,6 +139,7 @@ public:
     void synchronize();                                  // wait for the stream, then check_kernel_errors()
     void check_kernel_errors();                          // synchronises; throws KernelError when a kernel gave up on a wait
     void inject_error_word(int which, int code);         // for tests: as if a kernel had reported `code` (0 products, 1 attention)
+    bool stall_decode_stack(long long wait_cycles);      // for tests: DecodeStack::stall; false: this engine has none
     // After every run-order entry of the next steps, call `fn(entry index, residual [T, E] float32 with its
     // pending addend folded in, T, E)` with a host copy (for layer-by-layer comparison; turns graphs off while set).
     void set_layer_dump(std::function<void(int, const float*, int, int)> fn) { layer_dump_ = std::move(fn); }

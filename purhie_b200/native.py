@@ -201,6 +201,7 @@ _SIGNATURES = {
     "qe_engine_info": (c_char_p, [_P]),
     "qe_engine_cache_check": (c_int, [_P]),
     "qe_engine_set_error_word": (c_int, [_P, c_int, c_int]),
+    "qe_engine_stall_decode_stack": (c_int, [_P, c_longlong]),
     "qe_engine_set_layer_dump": (c_int, [_P, LAYER_DUMP_CB, c_void_p]),
     "qe_time_step": (c_int, [_P, POINTER(StepBatchC), POINTER(c_double)]),
     "qe_time_decode_steps": (c_int, [_P, POINTER(c_longlong), c_int, POINTER(c_int32), c_int, c_int, c_int, POINTER(c_double),

@@ -117,6 +117,7 @@ void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     a.part_o = ws.get("stack_part_o", {pieces, group, D}, DType::F32).as<float>();
     a.part_ml = ws.get("stack_part_ml", {pieces, group, 2}, DType::F32).as<float>();
     a.error_flag = ctx.attention_error;
+    a.wait_cycles = wait_cycles_;
     if (LaunchProfile::get().on()) {
         const double weights = (double)E * (first_.heads + 2 * first_.kv_heads) * D + (double)first_.heads * D * E + 3.0 * E * first_.inner;
         double keys = 0.0;
@@ -127,6 +128,13 @@ void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     const LayersKernels& k = layers_kernels();
     QE_LAUNCH(k, k.decode_layers(&a, ctx.stream));
     stream.clear();
+}
+
+void DecodeStack::stall(long long wait_cycles, cudaStream_t stream) {
+    wait_cycles_ = wait_cycles;
+    const int32_t first = wait_cycles ? -1 : 0;          // the counter of the first part; a launch leaves zeros
+    QE_CUDA(cudaMemcpyAsync(static_cast<int32_t*>(counters_.data()) + 1, &first, 4, cudaMemcpyHostToDevice, stream));
+    QE_CUDA(cudaStreamSynchronize(stream));
 }
 
 }  // namespace qe

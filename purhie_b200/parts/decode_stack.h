@@ -21,11 +21,14 @@ public:
     bool takes(const StepContext& ctx) const;
     // Every layer over the rows of stream.x, in place; nothing is pending afterwards.
     void run(ResidualStream& stream, StepContext& ctx) const;
+    // For tests: the next launch waits for a CTA that never reports, and every wait from now on ends after so many cycles (0: as usual,
+    // and nobody is waited for in vain).
+    void stall(long long wait_cycles, cudaStream_t stream);
 private:
     DecodeStack() = default;
     DecodeLayerSpec first_;
     int n_layers_ = 0, group_ = 0, page_size_ = 0, total_rows_ = 0, most_groups_ = 0, num_ctas_ = 0;
-    long long page_stride_ = 0;
+    long long page_stride_ = 0, wait_cycles_ = 0;
     DeviceBuffer layers_, maps_, shares_, counters_;
 };
 

@@ -114,3 +114,39 @@ def test_engines_one_after_the_other_read_their_own_weights_and_caches():
     for i in range(6):
         one, many = logits(i, 8 << i % 3, None), logits(i, 8 << i % 3, {"decode_stack": "off"})
         assert np.linalg.norm(one - many) < 0.03 * np.linalg.norm(many)
+
+
+def test_a_wait_that_runs_out_ends_the_launch_and_leaves_the_engine_usable():
+    """A CTA that never reports (its counter is held back): every wait ends after 20 million cycles, about ten milliseconds, the step
+    raises, and the next launch finds its counters as it needs them.  Rows whose keys several CTAs share, and K in chunks, so that
+    copies of every kind are on their way when the waits end."""
+    from purhie_b200 import native
+    from purhie_b200.engine import Engine, KernelError, StepEntry
+    config = _config(512, 4672, 6, 6, 2)
+    toks = random_tokens(800, config["vocab_size"], 3)
+
+    def engine():
+        return Engine.from_random(config, 3, dtype="bfloat16", max_tokens=8192, max_requests=4, cuda_graphs=False)
+
+    def logits(eng, names):
+        for r in names:
+            eng.add_request(r)
+            eng.step([StepEntry(r, toks[:700], [])])
+        out = [eng.step([StepEntry(r, toks[700 + k:701 + k], [0]) for r in names]).copy() for k in range(2)]
+        for r in names:
+            eng.release(r)
+        return np.stack(out)
+    eng, other = engine(), engine()
+    for r in "ab":
+        eng.add_request(r)
+        eng.step([StepEntry(r, toks[:700], [])])
+    for cycles in (20_000_000, 40_000_000):
+        native.check(native.lib().qe_engine_stall_decode_stack(eng.handle, cycles))
+        with pytest.raises(KernelError, match="one-launch decode step waited too long"):
+            eng.step([StepEntry(r, toks[700:701], [0]) for r in "ab"])
+    native.check(native.lib().qe_engine_stall_decode_stack(eng.handle, 0))
+    for r in "ab":
+        eng.release(r)
+    assert np.array_equal(logits(eng, "cde"), logits(other, "cde"))
+    eng.close()
+    other.close()
