@@ -383,15 +383,20 @@ int launch_rows_split(const float* x, const float* w, float* y, int M, int N, in
     return check_launch("gemm_simple");
 }
 
-// Columns a CTA takes: 8 while there are at most two such CTAs an SM, with K shared out among the warps where it has three blocks
-// or more (4 x 1024 x 3072: 8.4 us, 12.9 as one chain a thread; 8 x 1024 x 3072: 10.4 and 18.1; with one block seven of eight warps
-// would stand by); 32 with a row or a few per thread beyond; 64 for two to four rows of more columns than that is good for
-// (4 x 151936 x 1024, which streams 622 MB: 121 against 140 us).
+// Columns a CTA takes: 8 while there are at most two such CTAs an SM; 32 with a row or a few per thread beyond; 64 for two to four
+// rows of more columns than that is good for (4 x 151936 x 1024, which streams 622 MB: 121 against 140 us).  With 8, K is shared out
+// among the warps where it has three blocks or more (4 x 1024 x 3072: 8.4 us, 12.9 as one chain a thread; 8 x 1024 x 3072: 10.4 and
+// 18.1; with one block seven of eight warps would stand by).  A CTA of that form has an SM to itself, so more CTAs than SMs are two
+// rounds of it, and with 16 rows a warp has little of K at a time: those gain from a longer K only (us, a chain a thread and shared
+// out: 8 x 2048 x 384 3.98 and 5.19, x 768 6.9 and 6.7, x 6144 39.3 and 27.0; 4 x 2368 x 384 3.58 and 4.37, x 896 5.84 and 6.21,
+// x 1024 6.72 and 6.61; 16 x 1024 x 384 3.10 and 3.98, x 768 4.98 and 4.90).
 template <int MB>
 int plan_rows(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t stream) {
     const long long sms = multiprocessors();
     if (N <= 16 * sms) {
-        if (K > 2 * KC) return launch_rows_split<8, MB, MB <= 4 ? 1 : MB / 4, MB == 1 ? 4 : 8, MB == 4 ? 3 : 2>(x, w, y, M, N, K, stream);
+        const bool one_round = N <= 8 * sms && MB <= 8;
+        if (K > 2 * KC && (one_round || K >= (MB >= 8 ? 768 : 1024)))
+            return launch_rows_split<8, MB, MB <= 4 ? 1 : MB / 4, MB == 1 ? 4 : 8, MB == 4 ? 3 : 2>(x, w, y, M, N, K, stream);
         return launch_rows<8, MB, 1, MB <= 8 ? 10 : 8>(x, w, y, M, N, K, stream);
     }
     if constexpr (MB == 2 || MB == 4)
