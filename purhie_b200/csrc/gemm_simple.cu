@@ -421,11 +421,15 @@ int gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, cuda
     if (M <= 8) return plan_rows<8>(x, w, y, M, N, K, stream);
     if (M <= 16) return plan_rows<16>(x, w, y, M, N, K, stream);
     // An SM holds eight groups whatever the split.  Few tiles want every group at work on each of them (256 x 1024 x 3072: 61.6 us
-    // with four groups a tile, 66 with two, 72 with one; 256 x 6144 x 1024: 104.5, 98.5, 100.5; 517 x 6144 x 1024: 207, 195, 190; the
-    // tiles without a split of K took 73.9, 100.8 and 191.7).
+    // with four groups a tile, 66 with two, 72 with one).  Beyond, a tile of one group is two warps, so an odd number of them an SM
+    // leaves two of its four partitions idle at the end, and two groups a tile do not; else one group reads and adds less
+    // (x 1024 x 3072, us with one and with two: 608 rows, five tiles an SM, 147 and 139; 768, six, 152 and 161; 1024, seven, 191 and
+    // 184; 1184, eight, 197 and 210; 1536, eleven, 288 and 284; from thirteen on the odd numbers are level, and 2048, fourteen, takes
+    // 335 and 358).
     const long long sms = multiprocessors(), tiles = (long long)((M + TILE - 1) / TILE) * ((N + TILE - 1) / TILE);
     if (tiles <= 2 * sms && K > 2 * KC) return launch_tile<4>(x, w, y, M, N, K, stream);
-    if (tiles <= 16 * sms && K > KC) return launch_tile<2>(x, w, y, M, N, K, stream);
+    const long long most = (tiles + sms - 1) / sms;
+    if (most % 2 && most < 13 && K > KC) return launch_tile<2>(x, w, y, M, N, K, stream);
     return launch_tile<1>(x, w, y, M, N, K, stream);
 }
 

@@ -159,3 +159,8 @@ def product_us(M, N, K, dtype=torch.float32):
 def test_short_products_of_more_columns_than_a_round_holds_are_not_shared_out(M, N):
     """Half of K takes 0.59 and 0.47 of the time as a chain a thread, 0.78 and 0.74 with K shared out in two rounds."""
     assert product_us(M, N, 384) < 0.68 * product_us(M, N, 768)
+
+
+def test_tiles_of_one_group_where_their_number_an_sm_is_even():
+    """Fourteen tiles an SM take as long as thirteen with one group a tile, 1.07 times as long with two."""
+    assert product_us(2048, 1024, 3072) < 1.035 * product_us(1920, 1024, 3072)
