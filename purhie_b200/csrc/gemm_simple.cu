@@ -44,50 +44,58 @@ __global__ void __launch_bounds__(256) gemm_simple_kernel(const TX* __restrict__
     const int tid = threadIdx.x;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tr = tid / (BN / TN), tc = tid % (BN / TN);      // 16 x 16 threads
-    float total[TM][TN], acc[TM][TN][2];
+    float total[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) total[i][j] = acc[i][j][0] = acc[i][j][1] = 0.0f;
+        for (int j = 0; j < TN; ++j) total[i][j] = 0.0f;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 rows x 16 k = 1024 elements of each operand, 4 per thread
+    // 64 rows x 16 k = 1024 elements of each operand, 4 per thread, on their way while the 16 k in front of them are multiplied: few
+    // CTAs wait for little else (bfloat16, us with one chain an output, with blocks of K, and now: 1 x 4096 x 1020 185, 195 and 78;
+    // 512 x 4096 x 1020 317, 336 and 251; 1024 x 4096 x 1020 456, 480 and 434)
+    float xv[4], wv[4];
+    auto fetch = [&](int k0) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int idx = tid + e * 256;
-            const int r = idx / BK, kk = idx % BK;
-            const int k = k0 + kk;
-            float xv = 0.0f, wv = 0.0f;
-            if (k < K) {
-                if (m0 + r < M) xv = to_float<TX>(x[(size_t)(m0 + r) * K + k]);
-                if (n0 + r < N) wv = to_float<TW>(w[(size_t)(n0 + r) * K + k]);
+            const int r = (tid + e * 256) / BK, k = k0 + tid % BK;
+            xv[e] = k < K && m0 + r < M ? to_float<TX>(x[(size_t)(m0 + r) * K + k]) : 0.0f;
+            wv[e] = k < K && n0 + r < N ? to_float<TW>(w[(size_t)(n0 + r) * K + k]) : 0.0f;
+        }
+    };
+    fetch(0);
+    for (int block = 0; block < K; block += KC) {
+        float acc[TM][TN][2];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0f;
+        const int end = min(block + KC, K);
+        for (int k0 = block; k0 < end; k0 += BK) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                xs[tid % BK][(tid + e * 256) / BK] = xv[e];
+                ws[tid % BK][(tid + e * 256) / BK] = wv[e];
             }
-            xs[kk][r] = xv;
-            ws[kk][r] = wv;
+            __syncthreads();
+            fetch(k0 + BK);
+#pragma unroll
+            for (int kk = 0; kk < BK; ++kk) {
+                float a[TM], b[TN];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) a[i] = xs[kk][tr * TM + i];
+#pragma unroll
+                for (int j = 0; j < TN; ++j) b[j] = ws[kk][tc * TN + j];
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j][kk & 1] = fmaf(a[i], b[j], acc[i][j][kk & 1]);
+            }
+            __syncthreads();
         }
-        __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], b[TN];
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = xs[kk][tr * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = ws[kk][tc * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j][kk & 1] = fmaf(a[i], b[j], acc[i][j][kk & 1]);
-        }
-        if ((k0 + BK) % KC == 0 || k0 + BK >= K) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    total[i][j] += __fadd_rn(acc[i][j][0], acc[i][j][1]);
-                    acc[i][j][0] = acc[i][j][1] = 0.0f;
-                }
-        }
-        __syncthreads();
+            for (int j = 0; j < TN; ++j) total[i][j] += __fadd_rn(acc[i][j][0], acc[i][j][1]);
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {

@@ -164,3 +164,8 @@ def test_short_products_of_more_columns_than_a_round_holds_are_not_shared_out(M,
 def test_tiles_of_one_group_where_their_number_an_sm_is_even():
     """Fourteen tiles an SM take as long as thirteen with one group a tile, 1.07 times as long with two."""
     assert product_us(2048, 1024, 3072) < 1.035 * product_us(1920, 1024, 3072)
+
+
+def test_the_plain_kernel_waits_for_little_else_than_its_products():
+    """One row of a weight whose K no fast kernel takes: 0.31 of the time of 512 rows, 0.58 with a wait for memory at every 16 of K."""
+    assert product_us(1, 4096, 1020, torch.bfloat16) < 0.45 * product_us(512, 4096, 1020, torch.bfloat16)
