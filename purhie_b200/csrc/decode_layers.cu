@@ -61,7 +61,7 @@ constexpr int KEYS = 32;                        // keys of a stage
 constexpr int D = 128;
 constexpr int QPITCH = D * 2 + 16;
 constexpr int RED = 20;                         // floats between the tokens of a warp's 16 x 8 partial sums
-constexpr int PAGES = 1024;                     // page coordinates kept in shared memory
+constexpr int PAGES = 1024;                     // page coordinates kept in shared memory (DecodeStack asks for no more of 148 CTAs)
 constexpr int MAX_GROUP = 8;                    // query heads per kv head
 constexpr int PARTS = 5;                        // counters per layer
 constexpr int MERGE = 20;                       // pieces of a pair that are merged at once
@@ -86,6 +86,123 @@ struct Params {
 __host__ __device__ inline int segments(int k) { return (k + SEG - 1) / SEG; }
 // Segments of K whose rows are in shared memory at once: all of them, or halves of the places in turn.
 __host__ __device__ inline int chunk_of(int nseg, int slots) { return nseg <= slots ? nseg : slots / 2; }
+
+// How the blocks of keys of all (row, kv head) pairs are dealt, from the rows' lengths, the same by every CTA.  A piece costs its
+// blocks and about 13 more (5 us: queries, the chain of waits, what its warps and then its pair's pieces add up).
+//   Whole CTAs: a pair has CTAs of its own, more of them where a row is longer, and a CTA has one piece at most (0.6B shape, one row
+//   of 2,048: with pieces of two pairs in a CTA the others waited 5 us a layer for it).  A row gets whole multiples of the kv heads,
+//   so the largest piece can be far from the even share.
+//   Even shares: the pairs end to end, each as 13 and its blocks, cut into one range per CTA.  For rows that are long and do not
+//   divide well, or unequal (and for more pairs than CTAs).
+// The one with the shorter longest piece is taken.  us a layer with a launch per operation, with whole CTAs only, and now: width 2,048
+// with 16 kv heads, six rows of 2,048 70, 71 and 62, five of 8,192 106, 141 and 99, one of 32,768 beside seven of 256 110, 247 and 98;
+// 8B shape, seven rows of 8,192 130, 154 and 129, one of 32,768 beside seven of 256 158, 140 and 117.
+constexpr int PIECE = 13;
+// Most pieces of a pair: a merge asks for MERGE of them at once, twice a group's heads over two, each round about three blocks long
+// (16 heads over 2, one row of 2,048: 65.6 us a layer in 64 pieces, 47.6 in 20, a launch per operation 52.0).
+constexpr int ROUND = 3;
+__host__ __device__ inline int rounds_of(int parts, int group) { return parts > 1 ? (group * D + CONSUMERS - 1) / CONSUMERS * ((parts + MERGE - 1) / MERGE) : 0; }
+struct Deal {
+    int rows, kv_heads, ctas;
+    const int32_t *blocks, *before;             // per row: blocks of keys, first CTA (place, with even shares) of its pairs
+    int total;                                  // even shares: the length of all pairs end to end (0: whole CTAs)
+};
+struct Piece {
+    int row, head, b0, n, blocks;               // blocks b0 .. b0 + n - 1 of the pair's
+    int parts, index, first;                    // of the pair: its pieces, which one this is, the CTA of the first
+    int next;                                   // even shares: where the pair behind this begins
+};
+__host__ __device__ inline long long share_begin(const Deal& d, int cta) { return (long long)cta * d.total / d.ctas; }
+__host__ __device__ inline int share_of(const Deal& d, int at) { return (int)(((long long)(at + 1) * d.ctas - 1) / d.total); }
+// A CTA's i-th piece, asked for in order.
+__host__ __device__ inline bool piece_at(const Deal& d, int cta, int i, Piece& s) {
+    const int M = d.rows, HKV = d.kv_heads;
+    if (!d.total) {
+        if (i || cta >= d.before[M]) return false;
+        s.row = 0;
+        while (s.row + 1 < M && cta >= d.before[s.row + 1]) ++s.row;
+        s.blocks = d.blocks[s.row];
+        s.parts = (d.before[s.row + 1] - d.before[s.row]) / HKV;
+        const int rest = cta - d.before[s.row];
+        s.head = rest / s.parts;
+        s.index = rest - s.head * s.parts;
+        s.first = cta - s.index;
+        s.b0 = s.index * s.blocks / s.parts;
+        s.n = (s.index + 1) * s.blocks / s.parts - s.b0;
+        return true;
+    }
+    const int begin = (int)share_begin(d, cta), end = (int)share_begin(d, cta + 1);
+    if (!i) s.next = begin;
+    while (s.next < end) {
+        s.row = 0;
+        while (s.row + 1 < M && s.next >= d.before[s.row + 1]) ++s.row;
+        s.blocks = d.blocks[s.row];
+        const int length = PIECE + s.blocks;
+        s.head = (s.next - d.before[s.row]) / length;
+        const int pair = d.before[s.row] + s.head * length, keys = pair + PIECE;
+        s.b0 = begin > keys ? begin - keys : 0;
+        s.n = (end - keys < s.blocks ? end - keys : s.blocks) - s.b0;
+        s.next = pair + length;
+        if (s.n > 0) {
+            s.first = share_of(d, keys);
+            s.parts = share_of(d, keys + s.blocks - 1) - s.first + 1;
+            s.index = cta - s.first;
+            return true;
+        }
+    }
+    return false;
+}
+// Fills in `before` ([rows + 1]) from `blocks`; returns Deal::total.
+__host__ __device__ inline int deal_out(int M, int HKV, int group, int ctas, const int32_t* blocks, int32_t* before) {
+    int whole = 0x7fffffff;                                              // the longest piece with whole CTAs, in blocks
+    if (M * HKV <= ctas) {
+        // one CTA a pair, then the rest to the rows with the most blocks per CTA, as long as the merge does not eat it up
+        int used = M * HKV, parts[ROWS], most_parts[ROWS];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            int rounds = 1;
+            if (i < M)
+                while (blocks[i] > MERGE * rounds * (rounds + 1) * ROUND * rounds_of(2, group)) ++rounds;
+            parts[i] = 1;
+            most_parts[i] = MERGE * rounds;
+        }
+        while (used + HKV <= ctas) {
+            int best = -1, most = 1;
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i)
+                if (i < M && parts[i] < most_parts[i]) {
+                    const int per = (blocks[i] + parts[i] - 1) / parts[i];
+                    if (per > most) { most = per; best = i; }
+                }
+            if (best < 0) break;
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) parts[i] += i == best;
+            used += HKV;
+        }
+        int at = 0;
+        whole = 0;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+            if (i < M) {
+                before[i] = at;
+                at += parts[i] * HKV;
+                const int piece = (blocks[i] + parts[i] - 1) / parts[i] + ROUND * rounds_of(parts[i], group);
+                if (piece > whole) whole = piece;
+            }
+        before[M] = at;
+    }
+    int total = 0, longest = 0;
+    for (int i = 0; i < M; ++i) {
+        total += HKV * (PIECE + blocks[i]);
+        if (blocks[i] > longest) longest = blocks[i];
+    }
+    // (every share has a length, so every CTA between a pair's first and its last has a piece of it)
+    const int share = total / ctas;
+    if (share < 1 || whole <= share + ROUND * rounds_of(longest / share + 2, group)) return 0;
+    before[0] = 0;
+    for (int i = 0; i < M; ++i) before[i + 1] = before[i] + HKV * (PIECE + blocks[i]);
+    return total;
+}
 
 __device__ __forceinline__ void add_release(int32_t* p, int v) { asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 __device__ __forceinline__ int load_acquire(const int32_t* p) {
@@ -132,7 +249,7 @@ struct Cta {
     unsigned char *ring, *x;
     float *red, *acc, *fac;
     unsigned char *q_tile, *k_new, *v_new;
-    int32_t *z, *blocks, *before;               // per row: position, blocks of keys, first CTA of its pairs
+    int32_t *z, *blocks, *before;               // per row: position, blocks of keys, first CTA (place, with even shares) of its pairs
     int32_t* pages;
     PhDecodeLayer* layers;
     uint64_t *full, *empty, *x_full, *x_empty, *ready;
@@ -140,7 +257,7 @@ struct Cta {
     mutable bool gone;                          // ... and this thread knows: it neither waits nor frees places
     int* flag;
     int g0[4], ng[4];                           // this CTA's groups in each product
-    int sharers;                                // CTAs that have a piece of the attention (0: more pairs than CTAs)
+    Deal deal;
     bool attends;
 };
 
@@ -185,33 +302,6 @@ __device__ __forceinline__ void publish(int32_t* counter) {
     }
 }
 
-// A CTA's n-th piece of the attention: blocks b0 .. b0 + n - 1 of (row, kv head), the index-th of `parts` pieces of the pair.
-// With at least as many CTAs as pairs a pair has CTAs of its own, more of them where a row is longer, and a CTA has one piece
-// at most: the step of a pair is a chain of waits (queries, keys, merge), and a CTA with the end of one pair and the start of
-// the next walked it twice (0.6B shape, one row of 2,048: the others waited 5 us a layer for it).  Else whole pairs in turn.
-struct Piece { int row, head, b0, n, blocks, parts, index; };
-__device__ __forceinline__ bool piece_at(const Cta& c, const Params& p, int i, Piece& s) {
-    const int M = p.a.rows, HKV = p.a.kv_heads;
-    if (c.sharers) {
-        if (i || (int)blockIdx.x >= c.sharers) return false;
-        s.row = 0;
-        while (s.row + 1 < M && (int)blockIdx.x >= c.before[s.row + 1]) ++s.row;
-        s.blocks = c.blocks[s.row];
-        s.parts = (c.before[s.row + 1] - c.before[s.row]) / HKV;
-        const int rest = (int)blockIdx.x - c.before[s.row];
-        s.head = rest / s.parts;
-        s.index = rest - s.head * s.parts;
-        s.b0 = s.index * s.blocks / s.parts;
-        s.n = (s.index + 1) * s.blocks / s.parts - s.b0;
-        return true;
-    }
-    const int pair = (int)blockIdx.x + i * (int)gridDim.x;
-    if (pair >= M * HKV) return false;
-    s.row = pair / HKV; s.head = pair - s.row * HKV;
-    s.blocks = s.n = c.blocks[s.row];
-    s.parts = 1; s.index = s.b0 = 0;
-    return true;
-}
 __device__ __forceinline__ int page_row(const Cta& c, const Params& p, int row, int head, int block, int page) {
     const int pos = block * KEYS + (page << p.page_shift);
     if (pos > c.z[row]) return p.a.total_rows;                       // zeros
@@ -337,7 +427,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
     float* mine = red + (size_t)warp * G * RS;
     const int r0 = lane >> 2;
     Piece s;
-    for (int i = 0; piece_at(c, p, i, s); ++i) {
+    for (int i = 0; piece_at(c.deal, blockIdx.x, i, s); ++i) {
         const int z = c.z[s.row], pair = s.row * HKV + s.head;
         // (the rotation does not wait for the product in front)
         const int pos = min(max(p.a.rotation_positions[s.row], 0), p.a.max_position - 1);
@@ -462,7 +552,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
             if (s.parts == 1) {
                 ((__nv_bfloat16*)p.a.attn)[(size_t)s.row * HQ * D + (s.head * G + r) * D + d] = __float2bfloat16_rn(ll == 0.0f ? 0.0f : acc / ll);
             } else {
-                const size_t at = (size_t)blockIdx.x * G + r;
+                const size_t at = (size_t)(2 * blockIdx.x + (s.index == 0)) * G + r;     // (the end of one pair, the start of another)
                 p.a.part_o[at * D + d] = acc;
                 if (d == 0) *(float2*)(p.a.part_ml + at * 2) = make_float2(mm, ll);
             }
@@ -474,7 +564,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
             consumers_sync();
             if (*c.flag) {
                 // the last of the pair's CTAs: every reference and sum, and eight parts of the output, on their way at once
-                const size_t at = ((size_t)blockIdx.x - s.index) * G;
+                const size_t at = (size_t)2 * s.first * G;
                 for (int idx = threadIdx.x; idx < G * D; idx += CONSUMERS) {
                     const int r = idx / D, d = idx % D;
                     const float* po = p.a.part_o + (at + r) * D + d;
@@ -485,7 +575,7 @@ __device__ __forceinline__ void attention(const Cta& c, const Params& p, Ring& r
                         float v[MERGE];
 #pragma unroll
                         for (int u = 0; u < MERGE; ++u) {
-                            const int k = min(j + u, s.parts - 1) * G;
+                            const int part = min(j + u, s.parts - 1), k = (2 * part + (part == 0)) * G;
                             ml[u] = __ldcg(pml + k);
                             v[u] = __ldcg(po + (size_t)k * D);
                         }
@@ -555,31 +645,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
             c.z[i] = p.a.positions[i];
             c.blocks[i] = c.z[i] / KEYS + 1;
         }
-        // one CTA a pair, then the rest to the rows with the most blocks per CTA
-        int used = M * HKV, parts[ROWS];
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) parts[i] = 1;
-        while (used + HKV <= CTAS) {
-            int best = -1, most = 1;
-#pragma unroll
-            for (int i = 0; i < ROWS; ++i)
-                if (i < M) {
-                    const int per = (c.blocks[i] + parts[i] - 1) / parts[i];
-                    if (per > most) { most = per; best = i; }
-                }
-            if (best < 0) break;
-#pragma unroll
-            for (int i = 0; i < ROWS; ++i) parts[i] += i == best;
-            used += HKV;
-        }
-        int at = 0;
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-            if (i < M) {
-                c.before[i] = at;
-                at += parts[i] * HKV;
-            }
-        c.before[M] = at;
+        *c.flag = deal_out(M, HKV, p.a.heads / HKV, CTAS, c.blocks, c.before);
     }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
@@ -588,12 +654,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
         c.ng[w] = s[1] - s[0];
     }
     __syncthreads();
-    c.sharers = M * HKV <= CTAS ? c.before[M] : 0;
+    c.deal = Deal{M, HKV, CTAS, c.blocks, c.before, *c.flag};
     const int ppb = KEYS >> p.page_shift;                                // pages per block
     {
         Piece s;
-        c.attends = piece_at(c, p, 0, s);
-        for (int n = 0, at = 0; at < PAGES && piece_at(c, p, n, s); ++n, at += s.n * ppb)
+        c.attends = piece_at(c.deal, blockIdx.x, 0, s);
+        for (int n = 0, at = 0; at < PAGES && piece_at(c.deal, blockIdx.x, n, s); ++n, at += s.n * ppb)
             for (int i = threadIdx.x; i < s.n * ppb && at + i < PAGES; i += NTHREADS)
                 c.pages[at + i] = page_row(c, p, s.row, s.head, s.b0 + i / ppb, i % ppb);
     }
@@ -639,7 +705,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_layers_kernel(const Params
             auto keys = [&](const CUtensorMap* map) {
                 int at = 0;
                 Piece s;
-                for (int n = 0; piece_at(c, p, n, s); ++n)
+                for (int n = 0; piece_at(c.deal, blockIdx.x, n, s); ++n)
                     for (int j = 0; j < s.n; ++j) {
                         if (!fill(KEYS * D * 4)) return false;
                         for (int i = 0; i < ppb; ++i, ++at)
@@ -857,6 +923,27 @@ PH_EXPORT int ph_decode_layers_weight_map(void* out, const void* w, int rows, in
         return fail(PH_ERR_UNSUPPORTED, "decode_layers: the copy engine does not take a weight of %d x %d", rows, K);
     memcpy(out, &m, sizeof(m));
     return PH_OK;
+}
+
+// The deal of the keys for rows at these positions: nine numbers a piece (CTA, row, kv head, first block, blocks, the pair's blocks, its
+// pieces, which of them, the CTA of the first) to `out`, room for `most` pieces.  Returns how many there are.
+PH_EXPORT int ph_decode_layers_deal(int rows, int heads, int kv_heads, const int32_t* positions, int ctas, int32_t* out, int most) {
+    if (rows < 1 || rows > ROWS || kv_heads < 1 || heads < kv_heads || ctas < 1 || !positions || !out)
+        return fail(PH_ERR_ARG, "decode_layers: no deal of %d rows, %d heads over %d, to %d CTAs", rows, heads, kv_heads, ctas);
+    int32_t blocks[ROWS], before[ROWS + 1];
+    for (int i = 0; i < rows; ++i) blocks[i] = positions[i] / KEYS + 1;
+    const int total = deal_out(rows, kv_heads, heads / kv_heads, ctas, blocks, before);
+    const Deal d{rows, kv_heads, ctas, blocks, before, total};
+    int n = 0;
+    for (int cta = 0; cta < ctas; ++cta) {
+        Piece s;
+        for (int i = 0; piece_at(d, cta, i, s); ++i, ++n)
+            if (n < most) {
+                const int32_t v[9] = {cta, s.row, s.head, s.b0, s.n, s.blocks, s.parts, s.index, s.first};
+                memcpy(out + (size_t)n * 9, v, sizeof(v));
+            }
+    }
+    return n;
 }
 
 PH_EXPORT int ph_decode_layers_counters(int n_layers, int kv_heads) { return 2 + PARTS * n_layers + ROWS * kv_heads; }

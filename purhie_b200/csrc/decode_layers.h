@@ -41,8 +41,8 @@ struct PhDecodeLayersArgs {
     float* qkv;                        // [rows, (HQ + 2 HKV) 128]
     void* attn;                        // [rows, HQ 128] bfloat16
     void* act;                         // [rows, F] bfloat16
-    float* part_o;                     // [CTAs][HQ / HKV][128]
-    float* part_ml;                    // [CTAs][HQ / HKV][2]
+    float* part_o;                     // [2 CTAs][HQ / HKV][128]
+    float* part_ml;                    // [2 CTAs][HQ / HKV][2]
     int* error_flag;
     long long wait_cycles;             // limit of every wait (0: two seconds)
 };

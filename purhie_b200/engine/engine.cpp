@@ -406,6 +406,7 @@ Tensor Engine::step_graph(const std::vector<StepEntry>& entries, const int32_t* 
     std::string key = std::to_string(S) + "|" + std::to_string(ctx_bucket);
     for (int w : lay.widths) key += "|w" + std::to_string(w);
     for (const auto& a : lay.extra) key += "|" + a.first + ":" + std::to_string(a.second.second);
+    if (decode_stack_ && !decode_stack_->short_enough(lay.ctx_lens)) key += "|long";
     Graph* g = nullptr;
     for (auto it = graphs_.begin(); it != graphs_.end(); ++it)
         if (it->first == key) {

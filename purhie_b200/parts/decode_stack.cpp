@@ -55,6 +55,10 @@ std::unique_ptr<DecodeStack> DecodeStack::make(const std::vector<DecodeLayerSpec
     s->n_layers_ = (int)layers.size();
     s->group_ = v.group; s->page_size_ = v.page_size; s->page_stride_ = v.page_stride;
     s->num_ctas_ = sm_count();
+    // Every pair of eight rows a CTA of its own, at least: with more kv heads keys are most of a step, the attention kernel streams
+    // them 5 % faster than the ring does, and rows of 32,768 lost more than the launches cost (width 4,096 with 32 kv heads, us a layer
+    // with a launch per operation and with one: one row of 2,048 107 and 103, eight 144 and 155, one of 32,768 177 and 182).
+    if (a.kv_heads * kMostRows > s->num_ctas_) return nullptr;
     std::vector<int32_t> shares((size_t)4 * (s->num_ctas_ + 1));
     s->most_groups_ = k.shares((int)a.width, a.heads, a.kv_heads, (int)a.inner, s->num_ctas_, shares.data());
     if (uneven_us(shares, s->num_ctas_, a) > kMostUnevenUs) return nullptr;
@@ -80,8 +84,20 @@ std::unique_ptr<DecodeStack> DecodeStack::make(const std::vector<DecodeLayerSpec
     return s;
 }
 
+// Keys times kv heads of a step.  The ring streams keys at 5.8 TB/s and the attention kernel at 6.3, so beyond some 150 us of them a
+// layer what the launch saves is lost again: us a layer with a launch per operation and with one, 0.6B shape, five rows of 32,768
+// (1.3 million) 143 and 138, eight of 65,536 (4.2) 363 and 422; 8B shape, eight rows of 8,192 (0.5) 136 and 135, five of 32,768 195
+// and 198; width 2,048 with 16 kv heads, eight rows of 8,192 (1.05) 137 and 137, of 16,384 (2.1) 213 and 222.
+constexpr long long kMostKeys = 1 << 20;
+
+bool DecodeStack::short_enough(const std::vector<int>& lengths) const {
+    long long keys = 0;
+    for (int n : lengths) keys += n;
+    return keys * first_.kv_heads <= kMostKeys;
+}
+
 bool DecodeStack::takes(const StepContext& ctx) const {
-    if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T) return false;
+    if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T || !short_enough(ctx.ctx_lens)) return false;
     if (ctx.options && ctx.options->is_object() && !ctx.options->members().empty()) return false;
     return layers_kernels().supports(ctx.T, (int)first_.width, first_.heads, first_.kv_heads, first_.head_dim, (int)first_.inner, page_size_, n_layers_,
                                      most_groups_) != 0;
@@ -89,7 +105,7 @@ bool DecodeStack::takes(const StepContext& ctx) const {
 
 void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     const int T = ctx.T, group = first_.heads / first_.kv_heads;
-    const int64_t E = first_.width, D = first_.head_dim, pieces = num_ctas_;
+    const int64_t E = first_.width, D = first_.head_dim, pieces = 2 * num_ctas_;
     Workspace& ws = *ctx.workspace;
     const GroupStep& g = ctx.groups.at(group_);
     PhDecodeLayersArgs a{};

@@ -19,6 +19,8 @@ public:
     // Whether this step goes through the one launch.  The option "decode_stack": "off" keeps a launch per operation, and a step
     // with any other kernel choice among its options is made of the kernels it chooses.
     bool takes(const StepContext& ctx) const;
+    // The part of takes() that a step's lengths decide; a graph is captured for either answer.
+    bool short_enough(const std::vector<int>& lengths) const;
     // Every layer over the rows of stream.x, in place; nothing is pending afterwards.
     void run(ResidualStream& stream, StepContext& ctx) const;
     // For tests: the next launch waits for a CTA that never reports, and every wait from now on ends after so many cycles (0: as usual,

@@ -18,21 +18,24 @@ def _config(width, inner, heads, kv_heads, layers, vocab=640):
                 rope_theta=1e6, rms_norm_eps=1e-6, tie_word_embeddings=False, attention_bias=False)
 
 
-def _steps(folder, page_size, toks, prefixes, steps, options, graphs=True):
-    """Logits of every decoded token, [steps, rows, vocab], and whether the last step was a replay."""
+def _steps(folder, page_size, toks, prefixes, steps, options, graphs=True, max_tokens=8192):
+    """Logits of every decoded token, [steps, rows, vocab], whether the last step was a replay, and how many launches it had."""
+    from purhie_b200 import native
     from purhie_b200.engine import Engine, StepEntry
-    eng = Engine.from_folder(folder, dtype="bfloat16", page_size=page_size, max_tokens=8192, max_requests=len(prefixes), poison_cache=True,
+    eng = Engine.from_folder(folder, dtype="bfloat16", page_size=page_size, max_tokens=max_tokens, max_requests=len(prefixes), poison_cache=True,
                              cuda_graphs=graphs, step_options=options)
     out = []
     for r, n in enumerate(prefixes):
         eng.add_request(r)
-        if n:
-            eng.step([StepEntry(r, toks[r][:n], [])])
+        for at in range(0, n, 2048):
+            eng.step([StepEntry(r, toks[r][at:min(n, at + 2048)], [])])
     for k in range(steps):
+        before = native.lib().qe_launches()
         out.append(eng.step([StepEntry(r, toks[r][n + k:n + k + 1], [0]) for r, n in enumerate(prefixes)]).copy())
+    launches = native.lib().qe_launches() - before
     replayed = eng.last_stats.replayed_graph
     eng.close()
-    return np.stack(out), replayed
+    return np.stack(out), replayed, launches
 
 
 # width, inner, heads, kv heads, layers, page size, tokens in the cache per row
@@ -44,6 +47,9 @@ CASES = [
     (512, 4672, 6, 6, 2, 16, [5, 1500, 33, 0, 31, 32, 90, 1]),    # K in chunks through half of the places, with a ragged last one
     (2048, 6144, 8, 8, 2, 16, [1900]),                            # one row whose keys many CTAs share
     (1024, 17408, 8, 4, 1, 16, [40]),                             # one row, K longer than all places
+    (512, 320, 18, 18, 1, 16, [200, 33, 0, 64, 5, 100, 31, 32]),  # 144 (row, kv head) pairs, the most that are taken
+    (256, 128, 16, 16, 2, 16, [1500, 20, 20, 40, 20, 20, 20, 20]),    # a long row beside short ones: ends and starts of pairs in a CTA
+    (256, 128, 16, 2, 1, 32, [1900, 3]),                          # a pair whose pieces are merged in several rounds
 ]
 
 
@@ -56,10 +62,11 @@ def test_one_launch_gives_the_layers(width, inner, heads, kv_heads, layers, page
         pc, pw = P.read_model(tmp)
         toks = [random_tokens(n + steps, cfg.vocab_size, 11 + r) for r, n in enumerate(prefixes)]
         exact = np.stack([P.forward(pc, pw, t)[n:].numpy() for t, n in zip(toks, prefixes)], axis=1)
-        one, replayed = _steps(tmp, page_size, toks, prefixes, steps, None)
-        again, _ = _steps(tmp, page_size, toks, prefixes, steps, None, graphs=False)
-        many, _ = _steps(tmp, page_size, toks, prefixes, steps, {"decode_stack": "off"})
+        one, replayed, few = _steps(tmp, page_size, toks, prefixes, steps, None)
+        again, _, same = _steps(tmp, page_size, toks, prefixes, steps, None, graphs=False)
+        many, _, rest = _steps(tmp, page_size, toks, prefixes, steps, {"decode_stack": "off"})
     assert replayed
+    assert few == same <= 5 and rest >= few - 1 + 6 * layers      # embedding, layers, norm, output matrix (in two parts at most)
     assert np.array_equal(one, again)                             # nothing depends on the order in which CTAs arrive
     error = lambda got: np.linalg.norm((got - exact).ravel()) / np.linalg.norm(exact.ravel())
     # both forms round the same quantities to bfloat16 in the same places (normed rows, q, k, v, probabilities, heads,
@@ -68,9 +75,28 @@ def test_one_launch_gives_the_layers(width, inner, heads, kv_heads, layers, page
     assert error(one) < 0.02
 
 
+def test_steps_of_more_keys_than_the_launch_is_good_for():
+    """Two rows whose lengths cross 2^20 / 16 heads in the middle: one launch up to there and a launch per operation behind it, also as
+    graphs, which are captured for either."""
+    config = _config(64, 64, 16, 16, 1)
+    config["max_position_embeddings"] = 65536
+    prefixes = [32765, 32768]                                      # the third step has 65,537 + 2 keys
+    with tempfile.TemporaryDirectory() as tmp:
+        cfg = make_model(tmp, config, INIT, "bfloat16")
+        toks = [random_tokens(n + 4, cfg.vocab_size, 11 + r) for r, n in enumerate(prefixes)]
+        one, replayed, last = _steps(tmp, 8, toks, prefixes, 4, None, max_tokens=66000)
+        plain, _, again = _steps(tmp, 8, toks, prefixes, 4, None, graphs=False, max_tokens=66000)
+        first = _steps(tmp, 8, toks, prefixes, 1, None, graphs=False, max_tokens=66000)[2]
+        many, _, rest = _steps(tmp, 8, toks, prefixes, 4, {"decode_stack": "off"}, max_tokens=66000)
+    assert first < again == last == rest and replayed
+    assert np.array_equal(one, plain)
+    # the same quantities rounded to bfloat16 in the same places, in one layer
+    assert np.linalg.norm(one - many) < 0.01 * np.linalg.norm(many)
+
+
 def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
-    """Nine rows, a portion beside a decoded token, a step with a kernel choice and a width that divides badly are made of a launch
-    per operation."""
+    """Nine rows, a portion beside a decoded token, a step with a kernel choice, a width that divides badly and more kv heads than eight
+    rows have CTAs for are made of a launch per operation."""
     from purhie_b200 import native
     from purhie_b200.engine import Engine, StepEntry
     config = _config(256, 512, 4, 2, 3)
@@ -95,6 +121,7 @@ def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
         assert launches(rows, portion, options) > 3 * config["num_hidden_layers"]
     # 160 groups of 16 rows for 148 CTAs, twice a layer: the largest shares lose what the launches cost
     assert launches(1, False, None, _config(2560, 9728, 32, 8, 1)) > 3
+    assert launches(1, False, None, _config(256, 512, 20, 20, 1)) > 3
 
 
 def test_engines_one_after_the_other_read_their_own_weights_and_caches():
