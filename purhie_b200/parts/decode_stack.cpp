@@ -98,7 +98,9 @@ bool DecodeStack::short_enough(const std::vector<int>& lengths) const {
 
 bool DecodeStack::takes(const StepContext& ctx) const {
     if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T || !short_enough(ctx.ctx_lens)) return false;
-    if (ctx.options && ctx.options->is_object() && !ctx.options->members().empty()) return false;
+    if (ctx.option("decode_stack") == "off") return false;
+    for (const char* choice : {"decode_kernel", "decode_splits", "row_factor", "norm_ahead"})
+        if (ctx.options && ctx.options->find(choice)) return false;
     return layers_kernels().supports(ctx.T, (int)first_.width, first_.heads, first_.kv_heads, first_.head_dim, (int)first_.inner, page_size_, n_layers_,
                                      most_groups_) != 0;
 }

@@ -117,8 +117,11 @@ def test_rows_beyond_the_launch_and_chosen_kernels_take_the_other_path():
         eng.close()
         return n
     assert launches(1, False, None) == launches(8, False, None) == 2          # the embedding, the layers
-    for rows, portion, options in [(9, False, None), (3, True, None), (3, False, {"decode_kernel": "cp_async"}), (3, False, {"decode_stack": "off"})]:
-        assert launches(rows, portion, options) > 3 * config["num_hidden_layers"]
+    for options in [{"decode_stack": "on"}, {"prefill_kernel": "mma_sync"}, {"prefill_splits": 2}, {}]:
+        assert launches(3, False, options) == 2, options                      # choices that are not about such a step
+    for rows, portion, options in [(9, False, None), (3, True, None), (3, False, {"decode_kernel": "cp_async"}), (3, False, {"decode_splits": 2}),
+                                   (3, False, {"row_factor": "norm"}), (3, False, {"norm_ahead": "off"}), (3, False, {"decode_stack": "off"})]:
+        assert launches(rows, portion, options) > 3 * config["num_hidden_layers"], options
     # 160 groups of 16 rows for 148 CTAs, twice a layer: the largest shares lose what the launches cost
     assert launches(1, False, None, _config(2560, 9728, 32, 8, 1)) > 3
     assert launches(1, False, None, _config(256, 512, 20, 20, 1)) > 3
