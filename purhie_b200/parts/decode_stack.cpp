@@ -98,7 +98,8 @@ bool DecodeStack::short_enough(const std::vector<int>& lengths) const {
 
 bool DecodeStack::takes(const StepContext& ctx) const {
     if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T || !short_enough(ctx.ctx_lens)) return false;
-    if (ctx.option("decode_stack") == "off") return false;
+    // (a profile says what each operation takes, which one launch for all of them cannot)
+    if (LaunchProfile::get().on() || ctx.option("decode_stack") == "off") return false;
     for (const char* choice : {"decode_kernel", "decode_splits", "row_factor", "norm_ahead"})
         if (ctx.options && ctx.options->find(choice)) return false;
     return layers_kernels().supports(ctx.T, (int)first_.width, first_.heads, first_.kv_heads, first_.head_dim, (int)first_.inner, page_size_, n_layers_,
@@ -136,13 +137,6 @@ void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     a.part_ml = ws.get("stack_part_ml", {pieces, group, 2}, DType::F32).as<float>();
     a.error_flag = ctx.attention_error;
     a.wait_cycles = wait_cycles_;
-    if (LaunchProfile::get().on()) {
-        const double weights = (double)E * (first_.heads + 2 * first_.kv_heads) * D + (double)first_.heads * D * E + 3.0 * E * first_.inner;
-        double keys = 0.0;
-        for (int len : ctx.ctx_lens) keys += len;
-        LaunchProfile::get().note_cost(n_layers_ * (2.0 * weights + keys * 4.0 * first_.kv_heads * D),
-                                       n_layers_ * (2.0 * T * weights + keys * 4.0 * first_.heads * D));
-    }
     const LayersKernels& k = layers_kernels();
     QE_LAUNCH(k, k.decode_layers(&a, ctx.stream));
     stream.clear();

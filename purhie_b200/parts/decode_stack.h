@@ -17,7 +17,7 @@ public:
     // Null when the layers or the cache entries do not fit.
     static std::unique_ptr<DecodeStack> make(const std::vector<DecodeLayerSpec>& layers, const std::vector<CacheView>& views, cudaStream_t stream);
     // Whether this step goes through the one launch.  The option "decode_stack": "off" keeps a launch per operation, and so does a choice
-    // among the kernels that such a step is made of ("decode_kernel", "decode_splits", "row_factor", "norm_ahead").
+    // among the kernels that such a step is made of ("decode_kernel", "decode_splits", "row_factor", "norm_ahead"), and a profile.
     bool takes(const StepContext& ctx) const;
     // The part of takes() that a step's lengths decide; a graph is captured for either answer.
     bool short_enough(const std::vector<int>& lengths) const;

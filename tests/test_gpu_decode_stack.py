@@ -180,3 +180,23 @@ def test_a_wait_that_runs_out_ends_the_launch_and_leaves_the_engine_usable():
     assert np.array_equal(logits(eng, "cde"), logits(other, "cde"))
     eng.close()
     other.close()
+
+
+def test_a_profile_shows_the_operations_of_a_step():
+    from purhie_b200 import native
+    from purhie_b200.engine import Engine, StepEntry
+    config = _config(256, 512, 4, 2, 3)
+    toks = random_tokens(64, config["vocab_size"], 3)
+    eng = Engine.from_random(config, 3, dtype="bfloat16", max_tokens=1024, max_requests=1)
+    eng.add_request(0)
+    eng.step([StepEntry(0, toks[:20], [])])
+    native.lib().qe_profile_enable(1)
+    try:
+        native.profile_report()
+        eng.step([StepEntry(0, toks[20:21], [0])])
+        report = native.profile_report()
+    finally:
+        native.lib().qe_profile_enable(0)
+    eng.close()
+    assert "decode_layers" not in report and len(report) >= 6, report
+    assert any("attention" in name for name in report) and any("gemm" in name for name in report), report
