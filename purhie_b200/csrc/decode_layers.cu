@@ -946,6 +946,17 @@ PH_EXPORT int ph_decode_layers_deal(int rows, int heads, int kv_heads, const int
     return n;
 }
 
+// 1 if the current device takes cooperative launches and all `ctas` of them can be resident.
+PH_EXPORT int ph_decode_layers_resident(int ctas) {
+    int dev = 0, sms = 0, cooperative = 0, per_sm = 0;
+    const bool ok = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+                    cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess &&
+                    cudaFuncSetAttribute(decode_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_layers_kernel, NTHREADS, 227 * 1024) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok && cooperative && per_sm >= 1 && sms >= ctas ? 1 : 0;
+}
+
 PH_EXPORT int ph_decode_layers_counters(int n_layers, int kv_heads) { return 2 + PARTS * n_layers + ROWS * kv_heads; }
 
 // The copy engine's view of one cache entry, 128 bytes to `out` (host memory); as in attention_decode_bulk.cu.
@@ -1002,7 +1013,9 @@ PH_EXPORT int ph_decode_layers(const PhDecodeLayersArgs* args, cudaStream_t stre
     const cudaError_t e = cudaLaunchKernelEx(&cfg, decode_layers_kernel, p);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        return fail(PH_ERR_LAUNCH, "decode_layers: launch failed: %s", cudaGetErrorString(e));
+        // (a process may hold a part of the device only)
+        const bool refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported;
+        return fail(refused ? PH_LAYERS_REFUSED : PH_ERR_LAUNCH, "decode_layers: launch failed: %s", cudaGetErrorString(e));
     }
     return check_launch("decode_layers");
 }

@@ -15,6 +15,9 @@ struct PhDecodeLayer {
     void* v_base;
 };
 
+// ph_decode_layers: the device did not let all CTAs be resident at once; nothing was launched.
+#define PH_LAYERS_REFUSED 134
+
 struct PhDecodeLayersArgs {
     // fixed for a model and its cache
     const PhDecodeLayer* layers;       // [n_layers] on the device

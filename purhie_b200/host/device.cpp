@@ -283,6 +283,7 @@ const LayersKernels& layers_kernels() {
     void* h = open_library("layers");
     bind(h, "layers", "ph_decode_layers_supports", g_layers.supports);
     bind(h, "layers", "ph_decode_layers_shares", g_layers.shares);
+    bind(h, "layers", "ph_decode_layers_resident", g_layers.resident);
     bind(h, "layers", "ph_decode_layers_counters", g_layers.counters);
     bind(h, "layers", "ph_decode_layers_map", g_layers.map);
     bind(h, "layers", "ph_decode_layers_weight_map", g_layers.weight_map);

@@ -299,6 +299,7 @@ struct GemmKernels {
 struct LayersKernels {
     int (*supports)(int, int, int, int, int, int, int, int, int);
     int (*shares)(int, int, int, int, int, int32_t*);
+    int (*resident)(int);
     int (*counters)(int, int);
     int (*map)(void*, const void*, const void*, long long, int, int, int, int*);
     int (*weight_map)(void*, const void*, int, int);

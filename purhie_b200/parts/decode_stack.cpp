@@ -58,7 +58,7 @@ std::unique_ptr<DecodeStack> DecodeStack::make(const std::vector<DecodeLayerSpec
     // Every pair of eight rows a CTA of its own, at least: with more kv heads keys are most of a step, the attention kernel streams
     // them 5 % faster than the ring does, and rows of 32,768 lost more than the launches cost (width 4,096 with 32 kv heads, us a layer
     // with a launch per operation and with one: one row of 2,048 107 and 103, eight 144 and 155, one of 32,768 177 and 182).
-    if (a.kv_heads * kMostRows > s->num_ctas_) return nullptr;
+    if (a.kv_heads * kMostRows > s->num_ctas_ || !k.resident(s->num_ctas_)) return nullptr;
     std::vector<int32_t> shares((size_t)4 * (s->num_ctas_ + 1));
     s->most_groups_ = k.shares((int)a.width, a.heads, a.kv_heads, (int)a.inner, s->num_ctas_, shares.data());
     if (uneven_us(shares, s->num_ctas_, a) > kMostUnevenUs) return nullptr;
@@ -97,7 +97,7 @@ bool DecodeStack::short_enough(const std::vector<int>& lengths) const {
 }
 
 bool DecodeStack::takes(const StepContext& ctx) const {
-    if (!ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T || !short_enough(ctx.ctx_lens)) return false;
+    if (refused_ || !ctx.decode_only || ctx.T > kMostRows || ctx.T != ctx.S || ctx.n_decode_rows != ctx.T || !short_enough(ctx.ctx_lens)) return false;
     // (a profile says what each operation takes, which one launch for all of them cannot)
     if (LaunchProfile::get().on() || ctx.option("decode_stack") == "off") return false;
     for (const char* choice : {"decode_kernel", "decode_splits", "row_factor", "norm_ahead"})
@@ -106,7 +106,7 @@ bool DecodeStack::takes(const StepContext& ctx) const {
                                      most_groups_) != 0;
 }
 
-void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
+bool DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     const int T = ctx.T, group = first_.heads / first_.kv_heads;
     const int64_t E = first_.width, D = first_.head_dim, pieces = 2 * num_ctas_;
     Workspace& ws = *ctx.workspace;
@@ -138,13 +138,20 @@ void DecodeStack::run(ResidualStream& stream, StepContext& ctx) const {
     a.error_flag = ctx.attention_error;
     a.wait_cycles = wait_cycles_;
     const LayersKernels& k = layers_kernels();
-    QE_LAUNCH(k, k.decode_layers(&a, ctx.stream));
+    const int status = refuse_next_ ? PH_LAYERS_REFUSED : k.decode_layers(&a, ctx.stream);
+    if (status == PH_LAYERS_REFUSED) {
+        refused_ = true;                                  // and from now on a launch per operation
+        return false;
+    }
+    QE_LAUNCH(k, status);
     stream.clear();
+    return true;
 }
 
 void DecodeStack::stall(long long wait_cycles, cudaStream_t stream) {
-    wait_cycles_ = wait_cycles;
-    const int32_t first = wait_cycles ? -1 : 0;          // the counter of the first part; a launch leaves zeros
+    refuse_next_ = wait_cycles < 0;
+    wait_cycles_ = std::max(wait_cycles, 0ll);
+    const int32_t first = wait_cycles_ ? -1 : 0;          // the counter of the first part; a launch leaves zeros
     QE_CUDA(cudaMemcpyAsync(static_cast<int32_t*>(counters_.data()) + 1, &first, 4, cudaMemcpyHostToDevice, stream));
     QE_CUDA(cudaStreamSynchronize(stream));
 }

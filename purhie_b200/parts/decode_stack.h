@@ -21,16 +21,19 @@ public:
     bool takes(const StepContext& ctx) const;
     // The part of takes() that a step's lengths decide; a graph is captured for either answer.
     bool short_enough(const std::vector<int>& lengths) const;
-    // Every layer over the rows of stream.x, in place; nothing is pending afterwards.
-    void run(ResidualStream& stream, StepContext& ctx) const;
+    // Every layer over the rows of stream.x, in place; nothing is pending afterwards.  False: the device refused the launch (its CTAs
+    // must all be resident) and nothing was done; takes() says no from then on.
+    bool run(ResidualStream& stream, StepContext& ctx) const;
     // For tests: the next launch waits for a CTA that never reports, and every wait from now on ends after so many cycles (0: as usual,
-    // and nobody is waited for in vain).
+    // and nobody is waited for in vain; negative: as if the device refused the next launch).
     void stall(long long wait_cycles, cudaStream_t stream);
 private:
     DecodeStack() = default;
     DecodeLayerSpec first_;
     int n_layers_ = 0, group_ = 0, page_size_ = 0, total_rows_ = 0, most_groups_ = 0, num_ctas_ = 0;
     long long page_stride_ = 0, wait_cycles_ = 0;
+    bool refuse_next_ = false;
+    mutable bool refused_ = false;
     DeviceBuffer layers_, maps_, shares_, counters_;
 };
 

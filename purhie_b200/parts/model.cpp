@@ -116,8 +116,7 @@ Tensor DecoderModel::forward(StepContext& ctx, const std::vector<CacheView>& vie
         QE_CUDA(cudaMemcpyAsync(kept.data, stream.x.data, stream.x.bytes(), cudaMemcpyDeviceToDevice, ctx.stream));
         ctx.embedding_output = kept.as<float>();
     }
-    const bool one_launch = ctx.decode_stack && !after_entry && ctx.decode_stack->takes(ctx);
-    if (one_launch) ctx.decode_stack->run(stream, ctx);
+    const bool one_launch = ctx.decode_stack && !after_entry && ctx.decode_stack->takes(ctx) && ctx.decode_stack->run(stream, ctx);
     for (size_t i = 0; i < spec_.schedule.size() && !one_launch; i++) {
         ctx.pass = spec_.schedule[i].pass;
         // a layer learns which norm the next entry of the run order starts with: its last product may work ahead for it

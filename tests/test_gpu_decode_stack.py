@@ -199,4 +199,25 @@ def test_a_profile_shows_the_operations_of_a_step():
         native.lib().qe_profile_enable(0)
     eng.close()
     assert "decode_layers" not in report and len(report) >= 6, report
-    assert any("attention" in name for name in report) and any("gemm" in name for name in report), report
+    assert report["add_weight_sumsq"]["calls"] == 6, report         # the two norms of three layers
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_a_launch_that_the_device_refuses_is_made_of_operations(graphs):
+    """As where a process holds a part of the device only and the CTAs cannot all be resident: the step goes on with a launch per
+    operation, in the same engine, and so do the steps behind it."""
+    from purhie_b200 import native
+    from purhie_b200.engine import Engine, StepEntry
+    config = _config(256, 512, 4, 2, 3)
+    toks = random_tokens(64, config["vocab_size"], 3)
+
+    def logits(options, refuse):
+        eng = Engine.from_random(config, 3, dtype="bfloat16", max_tokens=1024, max_requests=1, cuda_graphs=graphs, step_options=options)
+        eng.add_request(0)
+        eng.step([StepEntry(0, toks[:20], [])])
+        if refuse:
+            native.check(native.lib().qe_engine_stall_decode_stack(eng.handle, -1))
+        out = [eng.step([StepEntry(0, toks[20 + k:21 + k], [0])]).copy() for k in range(3)]
+        eng.close()
+        return np.stack(out)
+    assert np.array_equal(logits(None, True), logits({"decode_stack": "off"}, False))
