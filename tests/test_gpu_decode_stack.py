@@ -221,3 +221,38 @@ def test_a_launch_that_the_device_refuses_is_made_of_operations(graphs):
         eng.close()
         return np.stack(out)
     assert np.array_equal(logits(None, True), logits({"decode_stack": "off"}, False))
+
+
+def test_engines_of_two_threads_step_at_once():
+    """Two launches that each want every SM: a cooperative launch starts whole or not at all, so neither waits for a CTA that the other
+    keeps out."""
+    import threading
+    from purhie_b200.engine import Engine, StepEntry
+    config = _config(512, 1024, 8, 4, 4)
+    toks = random_tokens(400, config["vocab_size"], 3)
+
+    def engine(seed):
+        eng = Engine.from_random(config, seed, dtype="bfloat16", max_tokens=4096, max_requests=2)
+        return eng
+
+    def run(eng, out):
+        for r in "ab":
+            eng.add_request(r)
+            eng.step([StepEntry(r, toks[:300], [])])
+        for k in range(60):
+            out.append(eng.step([StepEntry(r, toks[300 + k:301 + k], [0]) for r in "ab"]).copy())
+        for r in "ab":
+            eng.release(r)
+    engines = [engine(3), engine(4)]
+    alone, beside = [[], []], [[], []]
+    for eng, out in zip(engines, alone):
+        run(eng, out)
+    threads = [threading.Thread(target=run, args=pair) for pair in zip(engines, beside)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for eng in engines:
+        eng.close()
+    assert len(beside[0]) == len(beside[1]) == 60
+    assert np.array_equal(alone, beside)
