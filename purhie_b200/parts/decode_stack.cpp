@@ -16,9 +16,10 @@ DeviceBuffer upload(const void* host, size_t bytes, cudaStream_t stream) {
 }
 // The launches that a layer saves, about twelve microseconds, against what it loses where a product's groups do not divide among
 // the CTAs: each product waits for its largest share, which streams at 44 GB/s an SM.  us a layer at one and eight rows
-// behind 2,048 tokens, a launch per operation and one launch: 0.6B shape (loses 2.6) 38.8 / 51.0 and 28.1 / 40.6; width 2,048 (2.4) 51.4 /
-// 65.1 and 39.5 / 54.5; 8B shape (6.3) 90.2 / 104.4 and 84.2 / 100.3; width 2,560 with 32 heads (11.5) 65.4 / 78.2 and, two steps of
-// the kernel before, 63.2 / 79.1.
+// behind 2,048 tokens, a launch per operation and one launch: 0.6B shape (loses 2.6) 39.8 / 52.4 and 29.5 / 42.6; width 2,048 (2.4)
+// 49.2 / 62.1 and 38.2 / 51.5; 8B shape (6.3) 88.8 / 103.4 and 85.7 / 100.7; width 5,120 with 17,408 inner and 40 heads (18.5)
+// 133 / 150 and 144 / 168; with 25,600 and 64 (24.5) 187 / 207 and 194 / 218.  Width 2,560 with 32 heads (11.5) lies between and is
+// left out: 63.8 / 76.5 and 59.6 / 75.8, one to eight percent, which the form that the line was drawn for did not have.
 constexpr double kMostUnevenUs = 9.0;
 double uneven_us(const std::vector<int32_t>& shares, int ctas, const DecodeLayerSpec& a) {
     const double k[4] = {(double)a.width, (double)a.heads * a.head_dim, (double)a.width, (double)a.inner};
