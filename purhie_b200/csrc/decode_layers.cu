@@ -24,8 +24,8 @@
 // as one box per page as in attention_decode_bulk.cu; the step's own key and value are made by the CTA that holds the pair's last
 // block, which writes them to the cache and over their row of the stage.
 //
-// Measured (us a layer behind 2,048 tokens, a launch per operation -> this): 0.6B shape 38.8 -> 28.1 at one row, 51.0 -> 40.6 at eight;
-// width 2,048 51.4 -> 39.5 and 65.1 -> 54.5; 8B shape 90.2 -> 84.2 and 104.4 -> 100.3.  What bounds a layer now is the way of a
+// Measured (us a layer behind 2,048 tokens, a launch per operation -> this): 0.6B shape 38.9 -> 27.6 at one row, 51.1 -> 40.6 at eight;
+// width 2,048 48.1 -> 36.4 and 61.2 -> 50.1; 8B shape 86.2 -> 79.1 and 98.8 -> 92.6.  What bounds a layer now is the way of a
 // result to the other CTAs, five times: barrier and release 1.2 us, the poll 0.7, the rows' way to shared memory 1.2, and in the
 // attention twice that for the merge; with larger weights also the copying thread's turn (a stage in 390 ns, 42 GB/s an SM).
 //
